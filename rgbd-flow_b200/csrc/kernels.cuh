@@ -28,7 +28,10 @@ struct PairCtl {
     int level_done;               // k_control sets it when the outer early-termination test passes
     int sor_stop;                 // k_sor (the CTA of tile 0) sets it once a convergence check breaks
     int sor_stop_iter;            // iterations executed when the break happened
-    int pad0;
+    int x_stop;                   // register SOR (sor_regs.cuh): the ping-pong buffer the increment was left in
+    int x_in;                     // k_linearize: x_stop of the inner iteration before
+    int tiles_done;               // k_sor_fold: tiles folded in this outer iteration
+    unsigned arrived;             // k_sor_resident: CTAs that have reached a convergence check, over the checks
     unsigned maxdiff[kMaxChecks]; // k_sor: max |dx| of the checked iteration (float bits), per check
     // history (finest level = 0)
     int outer_exec[16];
@@ -62,12 +65,12 @@ struct LevelItem {
     T* x[2][3];                 // SOR increment, ping-pong pair
     T* sys[12];                 // compact linear system (see k_linearize)
     T* stat_part;               // per SOR tile partial of the early-termination statistic
-    int lin_tiles_x, lin_tile0; // linearisation / elementwise tiles: index base in the step's list
     int n_sor_tiles;            // SOR tiles (32 x 32 interior) of this item
     // coarser level (for the flow upsample); null at the coarsest level
     const T* uc[3];
     int Wc, Hc, pitch_c;
     T inv_ratio;                // 1 / pyramid ratio (u, v scale on upsample)
+    ulonglong2* exch;           // k_sor_resident's exchange words (two per element of a plane); null: not used
     // full-resolution info for the depth-magnitude quirk
     int xres_full;
     T f_full;
@@ -109,6 +112,7 @@ struct SorLaunch {
     int xout;          // whole-level kernel: ping-pong buffer that receives x (non-final inner iterations)
     int control;       // whole-level kernels: run the outer iteration's control after the fold (k_control's work)
     int n_checks;      // its convergence-check count
+    int masked;        // register kernels: the step is not finite, pixels outside the image are held at 0
 };
 
 template <class T, class S>
@@ -562,6 +566,10 @@ __global__ void k_level_setup(const LevelItem<T, S>* items, const Tile* tiles, i
     if (t.idx == 0 && threadIdx.x == 0) it.ctl->level_done = 0;
     if (i >= it.H || j >= it.W) return;
     const int W = it.W, H = it.H, l = i * W + j;
+    if (it.exch) {
+        const int x = cs_idx(i, j, it.hwp);
+        it.exch[x] = it.exch[(size_t)2 * it.hwp * H + x] = make_ulonglong2(0, 0);
+    }
     const T gf[5] = {(T)1 / 12, (T)-8 / 12, (T)0, (T)8 / 12, (T)-1 / 12};
     for (int f = 0; f < 2; f++) {
         const T* const* c = (const T* const*)(it.pyr + 3 * f);
@@ -653,11 +661,18 @@ k_linearize(const LevelItem<T, S>* items, const Tile* tiles, SolveConst<T> k, in
     PairCtl* ctl = it.ctl;
     if (ctl->level_done) return;
     if (t.idx == 0) {
-        if (threadIdx.x == 0) { ctl->sor_stop = 0; ctl->sor_stop_iter = -1; }
+        if (threadIdx.x == 0) {
+            ctl->sor_stop = 0;
+            ctl->sor_stop_iter = -1;
+            ctl->arrived = 0;
+            ctl->x_in = ctl->x_stop;
+        }
         for (int c = threadIdx.x; c < kMaxChecks; c += blockDim.x) ctl->maxdiff[c] = 0;
     }
     const int W = it.W, H = it.H;
     const int x0 = t.tx * LTW, y0 = t.ty * LTH;
+    // the increment of the inner iteration before: planes xsel, or (< 0) where the register kernels left it
+    const int xb = use_du ? (xsel < 0 ? ctl->x_stop : xsel) : 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typedef T Plane[LRH][LRW];
     Plane* sB = reinterpret_cast<Plane*>(smem_raw);  // [6] 0.4*I1 + 0.6*warped I2 (5 features + depth)
@@ -674,7 +689,7 @@ k_linearize(const LevelItem<T, S>* items, const Tile* tiles, SolveConst<T> k, in
         T U[3], D[3];
         for (int c = 0; c < 3; c++) {
             U[c] = it.u[c][lp];
-            D[c] = use_du ? it.x[xsel][c][cs_idx(gi, gj, it.hwp)] : (T)0;
+            D[c] = use_du ? it.x[xb][c][cs_idx(gi, gj, it.hwp)] : (T)0;
             sU[c][ry][rx] = U[c];
             sUD[c][ry][rx] = U[c] + D[c];
         }
@@ -723,6 +738,12 @@ k_linearize(const LevelItem<T, S>* items, const Tile* tiles, SolveConst<T> k, in
     __syncthreads();
     const int lx = tid % LTW, ly = tid / LTW;
     const int gi = y0 + ly, gj = x0 + lx;
+    if (gi < H && gj >= W && gj < 2 * it.hwp) {
+        // the half-rows' padding: the register SOR reads whole half-rows, and a pixel outside the image has
+        // a system of zeros
+        const int lp = cs_idx(gi, gj, it.hwp);
+        for (int c = 0; c < 12; c++) it.sys[c][lp] = (T)0;
+    }
     if (gi >= H || gj >= W) return;
     const int l = gi * W + gj;
     const int ry = ly + 2, rx = lx + 2;
@@ -846,10 +867,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// The update with the w row's neighbour coefficients (wL .. wD: edge weight times the depth-smoothness
+// weight of the edge's source pixel) given.
 template <class T>
-__device__ __forceinline__ void sor_point(const T* c, T aL, T aU, T aR, T aD, T sL, T sU, T s,
-                                          const T* xl, const T* xu, const T* xr, const T* xd, const T* xp,
-                                          T omega, T step, T* out)
+__device__ __forceinline__ void sor_point_w(const T* c, T aL, T aU, T aR, T aD, T wL, T wU, T wR, T wD,
+                                            const T* xl, const T* xu, const T* xr, const T* xd, const T* xp,
+                                            T omega, T step, T* out)
 {
     // Each row: v = (rhs - sum of neighbour terms - the other two unknowns' terms) / diag, relaxed
     // and clamped; every product-subtract is one fused multiply-add, in the reference's order.
@@ -870,14 +893,23 @@ __device__ __forceinline__ void sor_point(const T* c, T aL, T aU, T aR, T aD, T 
     v = mulR(v, c[1]);
     r = fmaR(omega, v, mulR(omc, xp[1]));
     out[1] = minT(maxT(r, subR(xp[1], step)), addR(xp[1], step));
-    // w row: neighbour coefficients carry the depth-smoothness weight of the edge's source pixel
-    v = -mulR(mulR(aL, sL), xl[2]);
-    v = fmaR(-mulR(aU, sU), xu[2], v); v = fmaR(-mulR(aR, s), xr[2], v); v = fmaR(-mulR(aD, s), xd[2], v);
+    // w row
+    v = -mulR(wL, xl[2]);
+    v = fmaR(-wU, xu[2], v); v = fmaR(-wR, xr[2], v); v = fmaR(-wD, xd[2], v);
     v = addR(v, c[8]);
     v = fmaR(-c[4], xp[0], v); v = fmaR(-c[5], xp[1], v);
     v = mulR(v, c[2]);
     r = fmaR(omega, v, mulR(omc, xp[2]));
     out[2] = minT(maxT(r, subR(xp[2], step)), addR(xp[2], step));
+}
+
+template <class T>
+__device__ __forceinline__ void sor_point(const T* c, T aL, T aU, T aR, T aD, T sL, T sU, T s,
+                                          const T* xl, const T* xu, const T* xr, const T* xd, const T* xp,
+                                          T omega, T step, T* out)
+{
+    sor_point_w<T>(c, aL, aU, aR, aD, mulR(aL, sL), mulR(aU, sU), mulR(aR, s), mulR(aD, s), xl, xu, xr, xd, xp, omega,
+                   step, out);
 }
 
 // Two same-colour neighbours of one row as one aligned vector access (even index).
@@ -1804,6 +1836,7 @@ k_sor_level_reg(const LevelItem<T, S>* items, const int* which, SolveConst<T> k,
             const int lc = cs_idx(gi, gj, hw);
             for (int v = 0; v < 3; v++) it.x[L.xout][v][lc] = xb[v * PLS + o];
         }
+        if (tid == 0) ctl->x_stop = L.xout;
     }
 }
 
@@ -2325,6 +2358,10 @@ __global__ void k_seam_load(const LevelItem<T, S>* items, const Tile* tiles, con
     if (i >= it.H || j >= it.W) return;
     const int W = it.W, H = it.H, l = i * W + j;
     const size_t N = (size_t)W * H;
+    if (it.exch) {
+        const int x = cs_idx(i, j, it.hwp);
+        it.exch[x] = it.exch[(size_t)2 * it.hwp * H + x] = make_ulonglong2(0, 0);
+    }
     for (int c = 0; c < 5; c++) {
         it.I1[c][l] = stS<S>((T)q.im1[(size_t)l * 5 + c]);
         it.I2[c][l] = stS<S>((T)q.im2[(size_t)l * 5 + c]);

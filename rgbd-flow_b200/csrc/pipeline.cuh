@@ -20,6 +20,7 @@
 
 #include "kernels.cuh"
 #include "hpb.cuh"
+#include "sor_regs.cuh"
 
 namespace rgbdflow {
 
@@ -144,6 +145,7 @@ struct HostParams {
     int sor_level;                            // whole-level SOR for levels that fit one CTA (0: off)
     int level_cluster;                        // > 1: such levels run on a cluster of this many CTAs instead
     int level_reg;                            // FP32 whole-level SOR with the system in registers (0: off)
+    int res_k;                                // iterations between the resident SOR's exchanges (0: resident_k())
 };
 
 // Row pitch of the u planes, and the checkerboard half-row length of the x / sys planes (16-byte
@@ -190,6 +192,7 @@ struct SorChoice {
     int ilp = 2;     // tile kernel lane mapping
     int seg = 0;     // strip band height (0: automatic)
     BandMap bands;   // explicit band layouts (strip_balanced_bands); strips of other heights use seg
+    int res_k = 0;         // resident SOR from registers, this many iterations between exchanges
     double us_per_it = 0;  // measured time per SOR iteration of the step
 };
 struct TuneTable {
@@ -220,6 +223,57 @@ static inline bool sor_tunable(const HostParams& hp)
     return hp.K == 0 && hp.sor_ilp == 0 && hp.sor_nbuf == 0 && hp.sor_strip == 1 && hp.strip_min_w == 0 &&
            hp.strip_min_h == 0 && hp.strip_seg == 0 && hp.strip_min_px == 0 && hp.strip_balanced == 0 &&
            hp.level_cluster == 0;
+}
+
+// Whether the solve's SOR runs from registers (sor_regs.cuh): FP32, nothing about the SOR asked for
+// explicitly and no override of the older kernels.  Measured against the fastest of the tile, strip and
+// whole-level cluster kernels on every level of 1 and 16 pairs: see k_sor_resident.
+template <class T>
+static inline bool sor_from_registers(const HostParams& hp)
+{
+    // the resident kernel's exchange tags number every iteration of a level
+    const double tags = (double)hp.n_outer * hp.n_inner * (hp.n_sor + 1.0);
+    return sizeof(T) == 4 && sor_tunable(hp) && hp.sor_level && hp.level_reg && tags < 2e9;
+}
+
+// Whether a level is small enough for one CTA with a position a thread (k_sor_level_reg), which beats the
+// resident kernel's four rows a warp there: 30 iterations of 40x30 41 us against 44, of 10x7 26 against 35.
+static inline bool whole_ok(int H, int hwp)
+{
+    return H * hwp <= kLevelRegMax && level_reg_smem_bytes<float>(H, hwp) <= 64 * 1024;
+}
+
+// The largest K <= kmax at which a level's tiles fit the launch's CTAs; 0: none does.
+static inline int resident_fit(int W, int H, int kmax, int ctas)
+{
+    for (int K = kmax; K >= 1; K--)
+        if (res_tiles(W, kResCols, K) * res_tiles(H, kResRows, K) <= ctas) return K;
+    return 0;
+}
+
+// Iterations between the exchanges of the resident SOR, for the items of one step: a larger K exchanges less
+// often but needs more CTAs (tiles overlap by 4 K), so fewer items run together.  The cost of a choice is
+// the sum over the groups of items that run together of their slowest item's time an iteration, with
+// the measured times of a half-sweep and an exchange.
+template <class X>
+static int resident_k(const std::vector<X>& items, const std::vector<int>& which, int ctas)
+{
+    int best = 1;
+    double best_cost = 1e30;
+    for (int K = 1; K <= kResMaxK; K++) {
+        double cost = 0, group = 0;
+        int used = 0;
+        for (int i : which) {
+            const int k = resident_fit(items[i].W, items[i].H, K, ctas);
+            const int n = res_tiles(items[i].W, kResCols, k) * res_tiles(items[i].H, kResRows, k);
+            if (used + n > ctas) { cost += group; group = 0; used = 0; }
+            used += n;
+            group = std::max(group, 2 * kResHalfSweep + (n > 1 ? kResExchange / k : 0.0));
+        }
+        cost += group;
+        if (cost <= best_cost) { best_cost = cost; best = K; }
+    }
+    return best;
 }
 
 // Items the autotuner may put on the strip kernel (FP32, at least two strips wide and two bands high).
@@ -485,6 +539,10 @@ struct Plan {
         int clus_c, clus_threads;
         size_t clus_smem;
         int clus_kp;  // > 0: the cluster items run on k_sor_level_cluster_reg with this many positions a thread
+        size_t res_items_off; int n_res;      // k_sor_resident: ResItem per item
+        int res_k, res_tiles;                 // iterations between exchanges, tiles of the step
+        int n_fold;                           // blocks of its fold (32 x 32 tiles)
+        bool regs;                            // the step's items all run from registers
     };
     std::vector<StepDesc> steps;
     struct PyrLevelDesc { size_t jobs_off; int n_jobs; size_t src_tiles_off; int n_src; size_t dst_tiles_off; int n_dst; size_t g_off; };
@@ -585,8 +643,8 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         }
     Bump A;
     P.ctl_off = A.take(sizeof(PairCtl) * P.n);
-    P.ctr_off = A.take(sizeof(int) * 16);
-    P.unfilled_off = A.take(sizeof(int) * 256 + sizeof(GridSync));
+    P.ctr_off = A.take(sizeof(int) * (16 + 256) + sizeof(GridSync));
+    P.unfilled_off = P.ctr_off + sizeof(int) * 16;
     {
         size_t nt = 0;
         for (const auto& p : pairs) nt += (size_t)((p.W + LTW - 1) / LTW) * ((p.H + LTH - 1) / LTH);
@@ -886,11 +944,9 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
             it.xres_full = (int)pairs[p].xres_full;
             it.f_full = (T)pairs[p].f_full;
             const int iid = (int)items.size();
-            it.lin_tiles_x = (it.W + LTW - 1) / LTW;
-            it.lin_tile0 = (int)lt.size();
-            const int lty = (it.H + LTH - 1) / LTH;
+            const int ltx = (it.W + LTW - 1) / LTW, lty = (it.H + LTH - 1) / LTH;
             for (int y = 0; y < lty; y++)
-                for (int x = 0; x < it.lin_tiles_x; x++) lt.push_back(Tile{iid, x, y, y * it.lin_tiles_x + x});
+                for (int x = 0; x < ltx; x++) lt.push_back(Tile{iid, x, y, y * ltx + x});
             items.push_back(it);
         }
         std::vector<int> strip_items, level_items, clus_items;
@@ -903,16 +959,41 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         // the tuned choice for this step's sizes, where the tuner has measured one
         const std::string skey = sor_step_key<T>(items);
         const SorChoice* ch = nullptr;
-        if (tune) {
+        // the step runs from registers when every item's level fits the device's
+        std::vector<size_t> scratch;
+        const int ctas = P.sms > 0 ? P.sms : 148;
+        bool regs = sor_from_registers<T>(hp);
+        for (size_t q = 0, p = 0; q < items.size(); q++, p++) {
+            while (k >= P.L[p]) p++;  // the item's pair
+            const auto& x = items[q];
+            // the exchange words live in the pair's full-resolution scratch (free once the pyramids are built)
+            const bool words = (size_t)4 * x.hwp * x.H * sizeof(ulonglong2) <= sizeof(T) * 10 * P.shapes[p].w[0] * P.shapes[p].h[0];
+            regs = regs && (whole_ok(x.H, x.hwp) || (words && resident_fit(x.W, x.H, 1, ctas) > 0));
+            scratch.push_back(l0[p].tmp);
+        }
+        if (tune && !regs) {
             const auto f = tune->m.find(skey);
             if (f != tune->m.end()) ch = &f->second;
         }
         P.step_keys.push_back(skey);
         P.step_tuned.push_back(ch != nullptr);
         const bool strips = ch ? ch->strip != 0 : strip_px >= (hp.strip_min_px > 0 ? hp.strip_min_px : 2000000L);
+        std::vector<int> res_items;
         for (auto& x : items) {
             const int sx = (x.W + kSorTW - 1) / kSorTW, sy = (x.H + kSorTH - 1) / kSorTH;
             x.n_sor_tiles = sx * sy;
+            if (regs) {
+                const int i = (int)(&x - items.data());
+                if (whole_ok(x.H, x.hwp)) {
+                    level_items.push_back(i);
+                    level_reg_smem = std::max(level_reg_smem, level_reg_smem_bytes<T>(x.H, x.hwp));
+                    level_thr = std::max(level_thr, level_threads(x.H, x.hwp));
+                    continue;
+                }
+                res_items.push_back(i);
+                x.exch = (ulonglong2*)scratch[i];
+                continue;
+            }
             if (use_level<T>(hp, x.W, x.H, x.hwp) && !(hp.level_cluster > 1 && x.H >= 2 * hp.level_cluster)) {
                 level_items.push_back((int)(&x - items.data()));
                 level_smem = std::max(level_smem, level_smem_bytes<T>(x.H, x.hwp));
@@ -983,6 +1064,37 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         d.clus_items_off = P.put(clus_items); d.n_clus = (int)clus_items.size();
         d.clus_c = clus_c; d.clus_smem = clus_smem; d.clus_threads = clus_thr;
         d.clus_kp = clus_reg ? reg_kp : 0;
+        // resident items, large ones first (small ones fill up what they leave of the CTAs)
+        std::stable_sort(res_items.begin(), res_items.end(),
+                         [&](int a, int b) { return (long)items[a].W * items[a].H > (long)items[b].W * items[b].H; });
+        std::vector<ResItem> ri;
+        d.regs = regs;
+        d.res_k = 0;
+        d.res_tiles = 0;
+        d.n_fold = 0;
+        if (!res_items.empty()) d.res_k = hp.res_k > 0 ? std::min(hp.res_k, kResMaxK) : resident_k(items, res_items, ctas);
+        for (int i : res_items) {
+            const auto& x = items[i];
+            ResItem m;
+            std::memset(&m, 0, sizeof(m));
+            m.ctl = x.ctl;
+            m.x = (float*)x.x[0][0];
+            m.exch = x.exch;
+            m.stride = (long long)(((size_t)x.x[0][1] - (size_t)x.x[0][0]) / sizeof(float));
+            for (int z = 0; z < 18; z++)
+                if ((size_t)(z < 6 ? x.x[z / 3][z % 3] : x.sys[z - 6]) != (size_t)m.x + sizeof(float) * m.stride * z)
+                    throw std::logic_error("increment and system planes not evenly spaced");
+            m.W = x.W; m.H = x.H; m.hw = x.hwp;
+            m.K = resident_fit(x.W, x.H, d.res_k, ctas);
+            m.nx = res_tiles(x.W, kResCols, m.K);
+            m.ny = res_tiles(x.H, kResRows, m.K);
+            d.res_tiles += m.nx * m.ny;
+            m.item = i;
+            m.fold0 = d.n_fold;
+            d.n_fold += x.n_sor_tiles;
+            ri.push_back(m);
+        }
+        d.res_items_off = P.put(ri); d.n_res = (int)ri.size();
         P.steps.push_back(d);
     }
     // output pointers (one per pair, in the order of the finest step's items = pair order)
@@ -990,14 +1102,14 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
     for (int p = 0; p < P.n; p++) outs.push_back((T*)P.out_pair_off[p]);
     P.out_ptrs_off = P.put(outs);
     std::vector<EstSrc> est(P.n);
-    std::vector<SeamSrc> seam(P.n);
+    std::vector<SeamSrc> seam(P.kind == 2 ? P.n : 0);
     for (int p = 0; p < P.n; p++) {
         const std::vector<size_t>& sg = P.in_seg[p];
         est[p].f = nullptr; est[p].d = nullptr;
         if (P.kind == 0 && pairs[p].est) est[p].f = (const float*)sg[4];
         if (P.kind == 1 && pairs[p].est_d) est[p].d = (const double*)sg[5];
-        std::memset(&seam[p], 0, sizeof(SeamSrc));
         if (P.kind == 2) {
+            std::memset(&seam[p], 0, sizeof(SeamSrc));
             seam[p].im1 = (const double*)sg[0]; seam[p].im2 = (const double*)sg[1];
             seam[p].dm1 = (const double*)sg[2]; seam[p].dm2 = (const double*)sg[3];
             seam[p].uvw = (const double*)sg[4];
@@ -1076,6 +1188,13 @@ static void bind_plan(Plan<T, S>& P, char* base)
             for (int c = 0; c < 12; c++) rebase(x.sys[c], base);
             rebase(x.stat_part, base);
             for (int c = 0; c < 3; c++) rebase_nz(x.uc[c], base);
+            rebase_nz(x.exch, base);
+        }
+        ResItem* ri = (ResItem*)(d + st.res_items_off);
+        for (int i = 0; i < st.n_res; i++) {
+            rebase(ri[i].ctl, base);
+            rebase(ri[i].x, base);
+            rebase(ri[i].exch, base);
         }
     }
     if (P.hpb) {
@@ -1109,6 +1228,7 @@ static void bind_plan(Plan<T, S>& P, char* base)
     SeamSrc* seam = (SeamSrc*)(d + P.seam_src_off);
     for (int p = 0; p < P.n; p++) {
         rebase_nz(est[p].f, base); rebase_nz(est[p].d, base);
+        if (P.kind != 2) continue;
         rebase_nz(seam[p].im1, base); rebase_nz(seam[p].im2, base); rebase_nz(seam[p].dm1, base);
         rebase_nz(seam[p].dm2, base); rebase_nz(seam[p].uvw, base); rebase_nz(seam[p].ddw, base);
         rebase_nz(seam[p].dsw, base); rebase_nz(seam[p].mag, base); rebase_nz(seam[p].regw, base);
@@ -1287,6 +1407,66 @@ template <class T> static inline bool sor_cfg_fits(const SorConfig& c)
     return sm <= 227 * 1024;
 }
 
+// Launches a cooperative kernel (every block resident: its blocks wait for one another).
+template <class K, class... A>
+static void launch_cooperative(K kernel, int grid, int block, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    RF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+// The SOR of inner iteration hh from registers: the whole-level items in one launch, the resident ones in
+// another (64 items at most), then (last inner iteration) their fold; both run the control.
+template <class T, class S>
+static int enqueue_sor_regs(const Plan<T, S>& P, char* base, int sidx, cudaStream_t st, const SolveConst<float>& k,
+                            int outer, int hh, Prof* pf)
+{
+    const auto& d = P.steps[sidx];
+    const LevelItem<T, S>* items = (const LevelItem<T, S>*)(base + P.desc_off + d.items_off);
+    const int lvl = P.Lmax - 1 - sidx, n_checks = P.n_checks[sidx].back();
+    const bool last = hh == P.hp.n_inner - 1;
+    int launches = 0;
+    SorLaunch L{};
+    L.nit = P.hp.n_sor; L.outer = outer;
+    L.xin_zero = hh == 0;
+    L.final_fold = last;
+    L.control = last;
+    L.n_checks = n_checks;
+    L.masked = !std::isfinite(k.step);
+    if (d.n_level) {
+        L.xin = hh & 1;
+        L.xout = L.xin ^ 1;
+        RF_PROF_B(pf, KC_SOR_LEVEL0 + lvl, st);
+        k_sor_level_reg<T, S><<<d.n_level, d.level_threads, d.level_smem, st>>>(
+            items, (const int*)(base + P.desc_off + d.level_items_off), k, L);
+        RF_PROF_E(pf, st);
+        launches++;
+    }
+    if (!d.n_res) return launches;
+    const ResItem* ri = (const ResItem*)(base + P.desc_off + d.res_items_off);
+    RF_PROF_B(pf, KC_SOR_LEVEL0 + lvl, st);
+    for (int i = 0; i < d.n_res; i += kResItems) {
+        launch_cooperative(k_sor_resident, std::min(P.sms, d.res_tiles), kResNT, st, ri + i, std::min(kResItems, d.n_res - i), k, L,
+                           (unsigned)(outer * P.hp.n_inner + hh) * (unsigned)(P.hp.n_sor + 1), P.status);
+        launches++;
+    }
+    if (last) {
+        k_sor_fold<S><<<d.n_fold, 512, 0, st>>>(items, ri, d.n_res, k, outer, n_checks);
+        launches++;
+    }
+    RF_PROF_E(pf, st);
+    return launches;
+}
+
 // The level loop of one step (sceneFlowSingleScale's outer / inner / SOR structure, .cu:755-954).
 template <class T, class S>
 static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t st, int setup, Prof* pf)
@@ -1314,13 +1494,13 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
         for (int hh = 0; hh < P.hp.n_inner; hh++) {
             const auto& sched = P.sor_sched[sidx][hh];
             // inner iterations after the first read the running increment (x of the previous SOR)
-            const int xsel = sched.front().xin;
+            const int xsel = d.regs ? -1 : sched.front().xin;
             RF_PROF_B(pf, KC_LIN, st);
             k_linearize<T, S><<<d.n_lin, LTW * LTH, lin_smem_bytes<T>(), st>>>(items, lt, k, hh > 0, xsel);
             RF_PROF_E(pf, st);
             launches++;
             const int lvl = P.Lmax - 1 - sidx;
-            if (d.n_level) {
+            if (d.n_level && !d.regs) {
                 // the whole-level items: every SOR iteration of this inner iteration in one launch
                 SorLaunch L{};
                 L.it0 = 0; L.nit = P.hp.n_sor; L.outer = outer;
@@ -1379,6 +1559,11 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
                 RF_PROF_E(pf, st);
                 launches++;
             }
+            if constexpr (sizeof(T) == 4)
+                if (d.regs) {
+                    launches += enqueue_sor_regs(P, base, sidx, st, k, outer, hh, pf);
+                    continue;
+                }
             for (SorLaunch L : sched) {
                 L.outer = outer;
                 L.seq = seq++;
@@ -1395,7 +1580,7 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
                 RF_PROF_E(pf, st);
             }
         }
-        if (!fold_control) {
+        if (!fold_control && !d.regs) {
             const int wpb = 4;
             RF_PROF_B(pf, KC_CTL, st);
             k_control<T, S><<<(d.n_items + wpb - 1) / wpb, 32 * wpb, 0, st>>>(items, d.n_items, k, outer,
@@ -1405,23 +1590,6 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
         }
     }
     return launches;
-}
-
-// Launches a cooperative kernel (every block resident: its blocks meet at grid barriers).
-template <class K, class... A>
-static void launch_cooperative(K kernel, int grid, int block, cudaStream_t st, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    RF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 // The HPB regularisation weights of every level (sceneFlowMultiscale.cpp:79-83, 114-116): the

@@ -190,6 +190,8 @@ HostParams host_params(const rgbdflow_params& p)
     h.level_cluster = e ? std::atoi(e) : 0;
     e = std::getenv("RGBDFLOW_LEVEL_REG");
     h.level_reg = e ? std::atoi(e) : 1;
+    e = std::getenv("RGBDFLOW_RESIDENT_K");
+    h.res_k = e ? std::atoi(e) : 0;
     h.fill_rounds = 253;  // round stamps are bytes: 0 valid, 1..253 rounds, 254 outside, 255 unfilled
     return h;
 }
@@ -233,8 +235,8 @@ std::string plan_key(const std::vector<PairSpec>& ps, const HostParams& hp, int 
                   hp.n_sor, hp.max_dist, hp.fill_holes, hp.fixed, hp.omega, hp.step, hp.eps_d, hp.eps_z, hp.eps_s,
                   hp.sor_tol, hp.outer_tol, hp.occ_margin, hp.occ_penalty, hp.max_grad, hp.period, hp.K * 100 + hp.sor_ilp * 10 + hp.sor_nbuf, hp.fill_rounds);
     k += buf;
-    std::snprintf(buf, sizeof buf, " strip %d %d %d %d %ld %d level %d %d %d", hp.sor_strip, hp.strip_min_w, hp.strip_min_h,
-                  hp.strip_seg, hp.strip_min_px, hp.strip_balanced, hp.sor_level, hp.level_cluster, hp.level_reg);
+    std::snprintf(buf, sizeof buf, " strip %d %d %d %d %ld %d level %d %d %d r %d", hp.sor_strip, hp.strip_min_w, hp.strip_min_h,
+                  hp.strip_seg, hp.strip_min_px, hp.strip_balanced, hp.sor_level, hp.level_cluster, hp.level_reg, hp.res_k);
     return k + buf;
 }
 
@@ -249,7 +251,9 @@ std::string topo_key(const Plan<T, S>& P, const HostParams& hp, int tag, bool de
     for (size_t i = 0; i < P.steps.size(); i++)
         k += std::to_string(P.steps[i].n_items > 0) + std::to_string(P.sor_cfg[i].K) + std::to_string(P.sor_cfg[i].nbuf) +
              std::to_string(P.sor_cfg[i].ilp) + (P.steps[i].n_sor > 0 ? "t" : "") + (P.steps[i].n_units > 0 ? "s" : "") +
-             (P.steps[i].n_level > 0 ? "l" : "") + (P.steps[i].n_clus > 0 ? "c" + std::to_string(P.steps[i].clus_c) + "r" + std::to_string(P.steps[i].clus_kp) : "") + ".";
+             (P.steps[i].n_level > 0 ? "l" : "") + (P.steps[i].regs ? "w" : "") +
+             (P.steps[i].n_res > 0 ? "r" + std::to_string((P.steps[i].n_res + kResItems - 1) / kResItems) : "") +
+             (P.steps[i].n_clus > 0 ? "c" + std::to_string(P.steps[i].clus_c) + "r" + std::to_string(P.steps[i].clus_kp) : "") + ".";
     const std::vector<PairSpec> none;
     return k + plan_key(none, hp, tag);
 }
@@ -475,6 +479,13 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
     std::vector<int> todo;
     for (int sidx = 0; sidx < P0.Lmax; sidx++)
         if (!P0.step_tuned[sidx] && (P0.steps[sidx].n_sor || P0.steps[sidx].n_units)) todo.push_back(sidx);
+    // the register SOR's steps go by rule (resident_k): recorded for the listing
+    for (int sidx = 0; sidx < P0.Lmax; sidx++) {
+        if (!P0.steps[sidx].regs) continue;
+        SorChoice ch;
+        ch.res_k = std::max(1, P0.steps[sidx].res_k);
+        tt.m["r" + P0.step_keys[sidx]] = ch;
+    }
     if (todo.empty()) {
         ts.complete[c->device & 63].insert(bkey);
         return;
@@ -1396,7 +1407,8 @@ int rgbdflow_autotune_describe(int device, char* buf, size_t len)
                 lay += " H" + std::to_string(e.first) + ":";
                 for (size_t q = 0; q < e.second.size(); q++) lay += (q ? "/" : "") + std::to_string(e.second[q]);
             }
-            if (ch.strip && !ch.bands.empty())
+            if (ch.res_k) std::snprintf(b, sizeof b, "%s registers, exchange every %d; ", kv.first.c_str() + 1, ch.res_k);
+            else if (ch.strip && !ch.bands.empty())
                 std::snprintf(b, sizeof b, "%s strip bands%s K %d %.2f us/it; ", kv.first.c_str(), lay.c_str(), ch.K, ch.us_per_it);
             else if (ch.strip) std::snprintf(b, sizeof b, "%s strip band %d K %d %.2f us/it; ", kv.first.c_str(), ch.seg, ch.K, ch.us_per_it);
             else std::snprintf(b, sizeof b, "%s tile K %d ilp %d %.2f us/it; ", kv.first.c_str(), ch.K, ch.ilp, ch.us_per_it);
