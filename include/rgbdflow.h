@@ -417,8 +417,8 @@ int rgbdflow_scene_flow_noalloc(const rgbdflow_pair* pair, const rgbdflow_params
  * (runFlowTwoFramesCeLiu, src/runFlowTwoFrames.cpp:30-45 -> OpticalFlow::Coarse2FineFlow,
  * src/opticalFlowMultiscale.cpp, with SmoothFlowSOR, src/SmoothFlowSOR.cpp).  The device solve
  * keeps the reference's FP64 arithmetic, operation order and lexicographic SOR order, so its flow
- * equals the reference's.  Its SOR runs as overlapping anti-diagonal sweeps in one thread block
- * per inner iteration, with sor_ring sweeps in flight.
+ * equals the reference's.  Its SOR runs as a pipeline of sweeps over the device's thread blocks; the
+ * device memory of a solve grows with sor_ring for images below 4096 pixels.
  * ------------------------------------------------------------------------------------------- */
 typedef struct rgbdflow_flow2d_params {
     double alpha;          /* smoothness weight (the demo's -s, 0.02) */
@@ -427,7 +427,7 @@ typedef struct rgbdflow_flow2d_params {
     int    n_outer;        /* outer fixed-point iterations at the finest level, + k at level k (10) */
     int    n_inner;        /* (1) */
     int    n_sor;          /* SOR iterations at the finest level, + 3 k at level k (400) */
-    int    sor_ring;       /* SOR sweeps in flight, 2..16 (8); the result does not depend on it */
+    int    sor_ring;       /* 2..16 (8): images the SOR's work space holds; the result does not depend on it */
 } rgbdflow_flow2d_params;
 
 /* The demo's values for flow type 1 (runFlowTwoFramesCeLiu, opticalFlowParams). */

@@ -6,28 +6,23 @@
 // its sweep changes the result by pixels on ordinary scenes.  So this solve keeps the
 // reference's arithmetic exactly: FP64, every operation rounded on its own (explicit __d*_rn
 // intrinsics, no fused multiply-adds), the reference's operation order, and its lexicographic
-// SOR order.  The SOR runs as anti-diagonal wavefronts: pixel (i, j) needs new values only from
-// diagonal i + j - 1 of its own sweep and old values from diagonal i + j + 1 of the previous
-// one, so one diagonal is a parallel step.  Consecutive sweeps overlap, each starting two steps
-// after the previous one; sweep s writes ring slot s % D and reads the previous sweep from slot
-// (s - 1) % D, and starts only after sweep s - D has finished without converging, so the slot of
-// the sweep that converges is never overwritten.
+// SOR order, run as a pipeline of sweeps (k_sor_pipeline).
 //
 // Data: planar FP64 per level; colour pyramids 3 channels interleaved (as DImage), features 5
 // channels interleaved.
 #pragma once
 #include <cuda_runtime.h>
-#include <cooperative_groups.h>
 
+#include <algorithm>
+#include <climits>
 #include <cmath>
-#include <vector>
+#include <cstdint>
 
 namespace rgbdflow {
 namespace f2d {
 
 constexpr int kThreads = 256;
-constexpr int kSorThreads = 1024;
-constexpr int kMaxRing = 16;
+constexpr int kMaxRing = 16;  // sor_ring's upper limit (accepted for callers that set it; nothing depends on it)
 constexpr int kMaxTaps = 64;
 
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
@@ -166,8 +161,8 @@ struct LevelBufs {
     double* warp;           // frame 2 features warped by the flow (5 channels)
     double *u, *v, *du, *dv, *phi;
     double *dxy, *dx2, *dy2, *dtdx, *dtdy;
-    double* coef;  // the SOR's per-pixel coefficients packed, 8 doubles a pixel: dxy, dx2, dy2,
-                   // dtdx, dtdy, phi (written by k_rhs; read-only during the SOR)
+    double2* coef; // the SOR's coefficients: four planes of W H pairs, each in diagonal order
+                   // (written by k_rhs; read-only during the SOR)
     int W, H;
 };
 
@@ -242,7 +237,27 @@ __device__ __forceinline__ double laplacian_phi(const double* x, const double* p
     return ddiv(out, ddiv(norm, (double)count));
 }
 
-// The right-hand sides (SmoothFlowSOR.cpp:144-151): -Itx - alpha * Lap(u), -Ity - alpha * Lap(v)
+// Diagonal order of a W x H image: diagonal d = i + j after diagonal, each by row.  The element of pixel
+// (i, d - i) is diag_base(d) + i.
+__host__ __device__ inline int diag_start(int d, int W, int H)
+{
+    const int a = W < H ? W : H, b = W < H ? H : W;
+    if (d <= 0) return 0;
+    if (d <= a) return d * (d + 1) / 2;
+    if (d <= b) return a * (a + 1) / 2 + (d - a) * a;
+    const int r = W + H - 1 - d;
+    return r <= 0 ? W * H : W * H - r * (r + 1) / 2;
+}
+__host__ __device__ inline int diag_base(int d, int W, int H)
+{
+    return diag_start(d, W, H) - (d - W + 1 > 0 ? d - W + 1 : 0);
+}
+
+// The right-hand sides (SmoothFlowSOR.cpp:144-151): -Itx - alpha * Lap(u), -Ity - alpha * Lap(v), and what an
+// SOR update (SmoothFlowSOR.cpp:166-215) reads of a pixel that no sweep changes: omega over the two
+// denominators (the reference divides anew at every update; same operands, same quotient) and the
+// neighbours' weights (0 where there is no neighbour).
+constexpr double kOmega = 1.8;
 __global__ void k_rhs(LevelBufs b, double alpha)
 {
     const int W = b.W, H = b.H;
@@ -251,288 +266,300 @@ __global__ void k_rhs(LevelBufs b, double alpha)
         const int i = (int)(p / W), j = (int)(p % W);
         const double tx = dsub(-b.dtdx[p], dmul(alpha, laplacian_phi(b.u, b.phi, W, H, i, j)));
         const double ty = dsub(-b.dtdy[p], dmul(alpha, laplacian_phi(b.v, b.phi, W, H, i, j)));
-        b.dtdx[p] = tx;
-        b.dtdy[p] = ty;
-        double4* c = reinterpret_cast<double4*>(b.coef + p * 8);
-        c[0] = make_double4(b.dxy[p], b.dx2[p], b.dy2[p], tx);
-        c[1] = make_double4(ty, b.phi[p], 0.0, 0.0);
+        const double phi = b.phi[p], phiL = j > 0 ? b.phi[p - 1] : 0.0, phiU = i > 0 ? b.phi[p - W] : 0.0;
+        double ws = 0;
+        if (j > 0) ws = dadd(ws, phiL);
+        if (j < W - 1) ws = dadd(ws, phi);
+        if (i > 0) ws = dadd(ws, phiU);
+        if (i < H - 1) ws = dadd(ws, phi);
+        ws = dmul(ws, alpha);
+        double2* c = b.coef + diag_base(i + j, W, H) + i;
+        c[0] = make_double2(b.dxy[p], ddiv(kOmega, dadd(b.dx2[p], ws)));
+        c[n] = make_double2(ddiv(kOmega, dadd(b.dy2[p], ws)), tx);
+        c[2 * n] = make_double2(ty, phi);
+        c[3 * n] = make_double2(phiU, phiL);
     }
 }
 
-// One SOR update (SmoothFlowSOR.cpp:166-215) of pixel (i, j): left / upper neighbours new (this
-// sweep's ring slot nw), right / lower neighbours and the pixel itself old (the previous sweep's
-// slot ow); a slot holds (du, dv) pairs.  Writes the new pair to nw and returns the change.
-template <bool CG = false>
-__device__ __forceinline__ double sor_update(const LevelBufs& b, double alpha, int i, int j, double2* nw,
-                                             const double2* ow)
+// ------------------------------------------------------------------------------------------
+// The SOR iterations of one inner iteration (SmoothFlowSOR.cpp:156-226): lexicographic sweeps with omega 1.8,
+// up to the first whose largest change is below 1e-5.  Pixel (i, j) of sweep s reads (i, j - 1) and
+// (i - 1, j) of its own sweep, and (i, j + 1), (i + 1, j) and itself of sweep s - 1.
+//
+// A task is G sweeps of a band; row l of the band is, in its sweep s, image row 32 B + l - s: rows move up by
+// one from sweep to sweep, so that all a row reads of sweep s - 1 lies in the band's rows l - 1 and l, and
+// data flows between bands in one direction.  A warp takes one sweep, a lane one of the band's 32 rows, each
+// lane one column behind the lane above: at step t lane l is at column t - l.  Then
+//   * the left neighbour is the lane's own last result, the upper one the lane above's (a shuffle),
+//   * the lower old value is what the warp of the sweep before put into its queue for this row, the right
+//     old one what it put there for the row above (a shuffle), the pixel's own old value the right one of
+//     the step before.
+// So an update reads one value of the sweep before and its coefficients; sweeps follow each other two steps
+// apart, a block barrier a step.  Values cross between tasks through L2: the band's last row, of each sweep,
+// to the band below, and the last sweep's image to the next G sweeps.  Those areas are filled with a
+// bit pattern that no operation produces (all ones) before the launch; two feeding warps poll the
+// values themselves.  Tasks are numbered so that a task reads only tasks before it; CTAs take them in order
+// (cooperative launch, every wait bounded).
+//
+// The largest change of each sweep is combined over the bands; the first sweep below 1e-5 is known once its
+// last band is done, and tasks of later sweeps stop.  When it is not its group's last sweep, a second
+// launch (finish) runs its group again with fewer sweeps: no result of a sweep after it is used.
+//
+// What bounds it: the step.  It is a chain of 15 dependent FP64 operations between two barriers, and a sweep
+// starts three steps after the one before it (two for the data, one for the rows' shift), so an inner
+// iteration of 400 sweeps is 1200 steps and the level's width and height.  Groups of 8 sweeps: 16 keep the FP64
+// pipe (2 cycles a warp instruction) longer in a step than its chain lasts, fewer have more hand-overs
+// through L2 and more tasks than SMs.  Measured, one solve, device time: 320x240 85.8 ms (16), 73.1 (12), 65.8 (8),
+// 67.4 (6), 67.8 (4); 160x120 46.6, 39.4, 34.9, 34.2, 34.0.  Diagonal after diagonal over a cluster of 16 CTAs, a
+// cluster barrier a step and every value through L2, it was 637 ms at 320x240.
+constexpr int kPipeG = 8, kPipeThreads = 32 * (kPipeG + 2), kPipeAhead = 4, kPipePolls = 1 << 20;
+
+struct PipeArgs {
+    int W, H, NB;                 // level, bands
+    int s0, n, G;                 // this launch's sweeps: the first, how many, in groups of G
+    double alpha;
+    const double2* coef;          // four planes of W H
+    double2* img;                 // images in diagonal order: slot 0 the input, slot g + 1 group g's, the last the finish's
+    double2* bnd;                 // last rows: [group, then the finish][band][sweep][column]
+    ulonglong2* sweep;            // of each of the launch's sweeps: largest change (bits), bands done
+    int* conv;                    // first sweep below the threshold (0x7f7f7f7f: none yet; -1: a wait gave up)
+    int zero_in;                  // the input is 0 (slot 0 is not read)
+    int finish;
+    int* status;                  // 1: a bounded wait gave up
+};
+
+__device__ __forceinline__ void pipe_store(double2* p, double2 v)
 {
-    // CG: the ring is written by other CTAs of a cluster; its values are read from L2
-    auto R = [](const double2* p) { return CG ? __ldcg(p) : *p; };
-    const int W = b.W, H = b.H;
-    const size_t o = (size_t)i * W + j;
-    const double omega = 1.8;
-    const double4 c0 = *reinterpret_cast<const double4*>(b.coef + o * 8);            // dxy, dx2, dy2, dtdx
-    const double2 c1 = __ldg(reinterpret_cast<const double2*>(b.coef + o * 8 + 4));  // dtdy, phi
-    const double phi = c1.y;
-    double sigmaU = 0, sigmaV = 0, weightSum = 0, w;
-    if (j > 0) {
-        w = __ldg(b.coef + (o - 1) * 8 + 5);
-        const double2 x = R(nw + o - 1);
-        sigmaU = dadd(sigmaU, dmul(w, x.x)); sigmaV = dadd(sigmaV, dmul(w, x.y)); weightSum = dadd(weightSum, w);
-    }
-    if (j < W - 1) {
-        w = phi;
-        const double2 x = R(ow + o + 1);
-        sigmaU = dadd(sigmaU, dmul(w, x.x)); sigmaV = dadd(sigmaV, dmul(w, x.y)); weightSum = dadd(weightSum, w);
-    }
-    if (i > 0) {
-        w = __ldg(b.coef + (o - W) * 8 + 5);
-        const double2 x = R(nw + o - W);
-        sigmaU = dadd(sigmaU, dmul(w, x.x)); sigmaV = dadd(sigmaV, dmul(w, x.y)); weightSum = dadd(weightSum, w);
-    }
-    if (i < H - 1) {
-        w = phi;
-        const double2 x = R(ow + o + W);
-        sigmaU = dadd(sigmaU, dmul(w, x.x)); sigmaV = dadd(sigmaV, dmul(w, x.y)); weightSum = dadd(weightSum, w);
-    }
-    sigmaU = dmul(sigmaU, -alpha);
-    sigmaV = dmul(sigmaV, -alpha);
-    weightSum = dmul(weightSum, alpha);
-    const double2 prev = R(ow + o);
-    const double prevDU = prev.x, prevDV = prev.y;
-    sigmaU = dadd(sigmaU, dmul(c0.x, prevDV));
-    const double nDU = dadd(dmul(1 - omega, prevDU), dmul(ddiv(omega, dadd(c0.y, weightSum)), dsub(c0.w, sigmaU)));
-    sigmaV = dadd(sigmaV, dmul(c0.x, nDU));
-    const double nDV = dadd(dmul(1 - omega, prevDV), dmul(ddiv(omega, dadd(c0.z, weightSum)), dsub(c1.x, sigmaV)));
-    nw[o] = make_double2(nDU, nDV);
-    return cmax(fabs(dsub(nDU, prevDU)), fabs(dsub(nDV, prevDV)));
+    asm volatile("{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(p),
+                 "l"(__double_as_longlong(v.x)), "l"(__double_as_longlong(v.y)) : "memory");
+}
+// Loads where `want` is set, 0 elsewhere (no branch: the loads of several steps are in flight together).
+__device__ __forceinline__ double2 pipe_load(const double2* p, bool want)
+{
+    unsigned long long lo, hi;
+    asm volatile("{\n .reg .pred w;\n .reg .b128 q;\n setp.ne.u32 w, %3, 0;\n mov.b128 q, {%4, %4};\n"
+                 " @w ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
+                 : "=l"(lo), "=l"(hi) : "l"(p), "r"((unsigned)want), "l"(0ull) : "memory");
+    return make_double2(__longlong_as_double(lo), __longlong_as_double(hi));
+}
+__device__ __forceinline__ bool pipe_ready(double2 v) { return __double_as_longlong(v.x) != -1LL; }
+// Brings a line of the coefficients into L1.
+__device__ __forceinline__ void pipe_touch(const double2* p)
+{
+    asm volatile("{\n .reg .f64 a, b;\n ld.global.ca.v2.f64 {a, b}, [%0];\n}\n" ::"l"(p));
 }
 
-// The step's work table, built by warp 0: for each sweep in flight (done + 1 .. next - 1, at most
-// 64), its diagonal and first row, and the prefix count of the step's items up to it (pre[0] = 0,
-// pre[n] = the step's items).  A sweep not on a diagonal of the level this step has no items.
-__device__ __forceinline__ void sor_table(int W, int H, long long t, int done, int next, const long long* start, int D,
-                                          int ndiag, int* pre, int* dd, int* ii0)
+__global__ void __launch_bounds__(kPipeThreads, 1) k_sor_pipeline(PipeArgs a)
 {
-    const int lane = threadIdx.x & 31;
-    const int n = next - (done + 1);
-    int run = 0;
-    for (int h = 0; h < 2; h++) {
-        const int l = lane + 32 * h;
-        int cnt = 0, d = 0, i0 = 0;
-        if (l < n) {
-            const long long dl = t - start[(done + 1 + l) % D];
-            if (dl >= 0 && dl < ndiag) {
-                d = (int)dl;
-                i0 = max(0, d - (W - 1));
-                cnt = min(H - 1, d) - i0 + 1;
-            }
-        }
-        int x = cnt;  // inclusive scan over the warp
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (l < n) {
-            pre[l + 1] = run + x;
-            dd[l] = d;
-            ii0[l] = i0;
-        }
-        run += __shfl_sync(0xffffffffu, x, 31);
-    }
-    if (lane == 0) pre[0] = 0;
-}
-
-// One step of the overlapping sweeps: for every sweep in flight, the pixels of its current
-// diagonal.  The step's updates are flattened into one list spread over the G threads (thread g
-// takes items g, g + G, ...), so the memory latency of the sweeps' updates overlaps across threads
-// instead of adding up sweep after sweep; an item finds its sweep in the step's table by binary
-// search.  Every update reads only values no other update of the step writes (the diagonal
-// structure), so the order within the step is free.
-template <bool CG>
-__device__ __forceinline__ void sor_step(const LevelBufs& b, double alpha, int done, int next, const int* pre,
-                                         const int* dd, const int* ii0, int D, size_t N, double2* ring,
-                                         unsigned long long* maxd, int g, int G)
-{
-    const int n = next - (done + 1);
-    const int total = n > 0 ? pre[n] : 0;
-    // whole warps iterate together (item k = kb + lane), so the sweeps' maxima can be combined
-    // per warp before the shared atomics
-    const int lane = threadIdx.x & 31;
-    for (int kb = g - lane; kb < total; kb += G) {
-        const int k = kb + lane;
-        int slot = -1;
-        unsigned long long bits = 0;
-        if (k < total) {
-            int lo = 0, hi = n - 1;  // the sweep l with pre[l] <= k < pre[l + 1]
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (pre[mid + 1] > k) hi = mid;
-                else lo = mid + 1;
-            }
-            const int s = done + 1 + lo;
-            const int i = ii0[lo] + (k - pre[lo]);
-            const int cur = s % D, prv = (s + D - 1) % D;
-            const double m = sor_update<CG>(b, alpha, i, dd[lo] - i, ring + (size_t)cur * N, ring + (size_t)prv * N);
-            if (m == m) {  // NaN is skipped, as std::max skips it
-                slot = cur;
-                bits = (unsigned long long)__double_as_longlong(m);  // ordered as the value (m >= 0)
-            }
-        }
-        // the largest change of each sweep among the warp's items (exact: the maximum of the
-        // 64-bit patterns, high word first), then one shared atomic per sweep and warp
-        const unsigned peers = __match_any_sync(0xffffffffu, slot);
-        const unsigned hi = __reduce_max_sync(peers, (unsigned)(bits >> 32));
-        const unsigned lo = __reduce_max_sync(peers, (unsigned)(bits >> 32) == hi ? (unsigned)bits : 0u);
-        if (slot >= 0 && lane == __ffs(peers) - 1) atomicMax(&maxd[slot], ((unsigned long long)hi << 32) | lo);
-    }
-}
-
-// The SOR iterations of one inner iteration (SmoothFlowSOR.cpp:156-226) as overlapping
-// anti-diagonal sweeps, one CTA.  ring: D slots of (u, v) increments, each N doubles.  Leaves the
-// last sweep's increments (the first that converged, max change < 1e-5, or sweep nSOR - 1) in
-// (du, dv) and the number of sweeps run in *sweeps.  status: 0, or 1 when the step bound ran out.
-__global__ void __launch_bounds__(kSorThreads) k_sor_wavefront(LevelBufs b, double alpha, int nSOR, int D,
-                                                               double2* ring, int* sweeps, int* status)
-{
-    const int W = b.W, H = b.H, ndiag = W + H - 1, lag = 2;
-    const size_t N = (size_t)W * H;
-    __shared__ long long start[kMaxRing];
-    __shared__ unsigned long long maxd[kMaxRing];
-    __shared__ int s_done, s_stop, s_next;
-    __shared__ int pre[kMaxRing + 1], dd[kMaxRing], ii0[kMaxRing];
-    for (size_t p = threadIdx.x; p < N; p += blockDim.x) {
-        ring[(size_t)(D - 1) * N + p] = make_double2(0.0, 0.0);
-    }
-    if (threadIdx.x == 0) { s_done = -1; s_stop = -1; s_next = 0; }
+    __shared__ double2 queue[kPipeG + 1][4][32];  // [sweep + 1 (0: the group's input)][step & 3][row]
+    __shared__ double2 edge[kPipeG + 1][4];       // the band above's last row: [sweep + 1][column & 3]
+    __shared__ int s_conv;
+    const int W = a.W, H = a.H, N = W * H, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int ng = (a.n + a.G - 1) / a.G;
+    int t0 = 0, t1 = ng * a.NB, gs_finish = 0;
+    if (tid == 0) s_conv = *(volatile int*)a.conv;
     __syncthreads();
-    // every sweep takes ndiag steps and starts within ndiag + lag steps of the previous one
-    const long long t_max = (long long)nSOR * (ndiag + lag) + ndiag + 8;
-    long long t = 0;
-    for (; t < t_max; t++) {
-        if (threadIdx.x < 32) {
-            // warp 0: the step's new sweep (lane 0), then the step's table
-            if (threadIdx.x == 0) {
-                const int nx = s_next;
-                if (nx < nSOR && (nx == 0 || t >= start[(nx - 1) % D] + lag) && (nx < D || s_done >= nx - D)) {
-                    start[nx % D] = t;
-                    maxd[nx % D] = 0ull;
-                    s_next = nx + 1;
+    const int conv0 = s_conv;
+    if (conv0 < a.s0) return;
+    if (a.finish) {
+        if (conv0 >= a.s0 + a.n) return;
+        const int g = (conv0 - a.s0) / a.G;
+        gs_finish = (conv0 - a.s0) % a.G + 1;
+        if (gs_finish == min(a.G, a.n - g * a.G)) return;  // the group's own image is the result
+        t0 = g * a.NB;
+        t1 = t0 + a.NB;
+    }
+    for (int task = t0 + blockIdx.x; task < t1; task += gridDim.x) {
+        const int g = task / a.NB, B = task % a.NB, slot = a.finish ? ng : g;
+        const int gs = a.finish ? gs_finish : min(a.G, a.n - g * a.G);
+        const double2* const in = a.img + (size_t)g * N;
+        double2* const out = a.img + (size_t)(slot + 1) * N;
+        double2* const bout = a.bnd + ((size_t)slot * a.NB + B) * a.G * W;
+        const double2* const bin = bout - (size_t)a.G * W;  // the band above's (not read by band 0)
+        const bool zero = a.zero_in && g == 0;
+        const int last = W + 30 + 2 * (gs - 1);             // the last step
+        bool stop = false, gave_up = false;
+        __syncthreads();  // every warp has left the last task's queues
+        if (w < kPipeG) {
+            // ---- sweep w of the group
+            const int row = 32 * B + lane - w;
+            const bool rowok = w < gs && row >= 0 && row < H;
+            double2 left = make_double2(0, 0), self = make_double2(0, 0);
+            double2 c[2][4] = {};
+            double mx = 0;
+            // the diagonal of the coefficients that are read next: at first that of tau = 0
+            int d = 32 * B - w, base = diag_base(d, W, H);
+            auto load_coef = [&](double2* q, int j) {
+                const bool ok = rowok && j >= 0 && j < W;
+                const double2* p = a.coef + (ok ? base + row : 0);
+#pragma unroll
+                for (int z = 0; z < 4; z++) q[z] = ok ? __ldg(p + (size_t)z * N) : make_double2(0, 0);
+                // to the next diagonal: past this one's elements, its first row one lower from column W - 1 on
+                if (d >= 0 && d < W + H - 1) base += min(H - 1, d) - max(0, d - W + 1) + 1 - (d + 1 - W + 1 > 0 ? 1 : 0);
+                d++;
+            };
+            if (__syncthreads_or(0)) stop = true;  // the feeding warps' first values are in place
+            for (int t = -1; !stop && t <= last; t += 2) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int tt = t + h, tau = tt - 2 * w, j = tau - lane;
+                    if (stop || tt > last) break;
+                    if (w < gs && tau >= -1 && tau <= W + 30) {
+                        double2 cc[4];
+#pragma unroll
+                        for (int z = 0; z < 4; z++) cc[z] = c[h][z];
+                        load_coef(c[h ^ 1], j + 1);
+                        const bool ok = rowok && j >= 0 && j < W;
+                        double2 lo = make_double2(0, 0);
+                        if (tau >= 0) lo = queue[w][tau & 3][lane];
+                        double2 right, up;
+                        right.x = __shfl_up_sync(0xffffffffu, lo.x, 1);
+                        right.y = __shfl_up_sync(0xffffffffu, lo.y, 1);
+                        up.x = __shfl_up_sync(0xffffffffu, left.x, 1);
+                        up.y = __shfl_up_sync(0xffffffffu, left.y, 1);
+                        if (lane == 0) {
+                            right = edge[w][(tau + 1) & 3];
+                            up = tau >= 0 ? edge[w + 1][tau & 3] : make_double2(0, 0);
+                        }
+                        const double dxy = cc[0].x, rU = cc[0].y, rV = cc[1].x, tx = cc[1].y, ty = cc[2].x, phi = cc[2].y;
+                        const double wL = cc[3].y, wU = cc[3].x, wR = j < W - 1 ? phi : 0.0, wD = row < H - 1 ? phi : 0.0;
+                        double sU = dadd(0.0, dmul(wL, left.x)), sV = dadd(0.0, dmul(wL, left.y));
+                        sU = dadd(sU, dmul(wR, right.x)); sV = dadd(sV, dmul(wR, right.y));
+                        sU = dadd(sU, dmul(wU, up.x)); sV = dadd(sV, dmul(wU, up.y));
+                        sU = dadd(sU, dmul(wD, lo.x)); sV = dadd(sV, dmul(wD, lo.y));
+                        sU = dadd(dmul(sU, -a.alpha), dmul(dxy, self.y));
+                        sV = dmul(sV, -a.alpha);
+                        const double nU = dadd(dmul(1 - kOmega, self.x), dmul(rU, dsub(tx, sU)));
+                        sV = dadd(sV, dmul(dxy, nU));
+                        const double nV = dadd(dmul(1 - kOmega, self.y), dmul(rV, dsub(ty, sV)));
+                        const double m = cmax(fabs(dsub(nU, self.x)), fabs(dsub(nV, self.y)));
+                        if (ok && m > mx) mx = m;  // a NaN is skipped, as std::max skips it
+                        left = ok ? make_double2(nU, nV) : make_double2(0, 0);
+                        self = right;
+                        if (tau >= 0) queue[w + 1][tau & 3][lane] = left;
+                        if (ok && lane == 31) pipe_store(bout + (size_t)w * W + j, left);
+                        if (ok && w == gs - 1) pipe_store(out + diag_base(row + j, W, H) + row, left);
+                    }
+                    if (__syncthreads_or(0)) stop = true;
                 }
             }
-            __syncwarp();
-            sor_table(W, H, t, s_done, s_next, start, D, ndiag, pre, dd, ii0);
-        }
-        __syncthreads();
-        const int done = s_done, next = s_next;
-        if (s_stop >= 0 || done >= nSOR - 1) break;
-        sor_step<false>(b, alpha, done, next, pre, dd, ii0, D, N, ring, maxd, threadIdx.x, blockDim.x);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            while (s_done + 1 < s_next && t - start[(s_done + 1) % D] == ndiag - 1) {
-                s_done++;
-                if (__longlong_as_double((long long)maxd[s_done % D]) < 1e-5) {
-                    s_stop = s_done;
-                    break;
+            if (!stop && w < gs && !a.finish) {
+                // bits of a double >= 0 order as the value
+                unsigned long long bits = (unsigned long long)__double_as_longlong(mx);
+                for (int o = 16; o; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
+                if (lane == 0) {
+                    const int s = g * a.G + w;
+                    ulonglong2* const sw = a.sweep + s;
+                    if (bits) atomicMax(&sw->x, bits);
+                    __threadfence();
+                    if (atomicAdd(&sw->y, 1ull) == (unsigned long long)(a.NB - 1)) {
+                        __threadfence();
+                        if (__longlong_as_double((long long)__ldcg(&sw->x)) < 1e-5) atomicMin(a.conv, a.s0 + s);
+                    }
+                }
+            }
+        } else {
+            // ---- the feeding warps.  Warp kPipeG: the group's input for the band's rows (image rows 32 B + lane + 1),
+            // column t + 1 - lane.  The next: lanes 0..G the band above's last row of sweep lane - 1 (lane 0:
+            // the input's row 32 B), column t + 1 - 2 (lane - 1)
+            const bool image = w == kPipeG;
+            const int q = lane - 1, row = image ? 32 * B + lane + 1 : 32 * B - 1 - q;
+            const bool from_image = image || lane == 0;
+            const bool rowok = row >= 0 && row < H && (from_image ? !zero : (B > 0 && lane <= gs));
+            auto col = [&](int t) { return image ? t + 1 - lane : t + 1 - 2 * q; };
+            auto wants = [&](int t) { const int c = col(t); return rowok && c >= 0 && c < W; };
+            auto at = [&](int t) {
+                const int c = col(t);
+                if (!wants(t)) return (const double2*)a.coef;
+                return from_image ? in + diag_base(row + c, W, H) + row : bin + (size_t)q * W + c;
+            };
+            auto poll = [&](int t, double2 v) {
+                for (int k = 0; !pipe_ready(v); k++) {
+                    if (k >= kPipePolls) { gave_up = true; break; }
+                    if ((k & 15) == 15 && *(volatile int*)a.conv < (a.finish ? 0 : a.s0 + g * a.G)) { stop = true; break; }
+                    v = pipe_load(at(t), true);
+                }
+                return v;
+            };
+            // the coefficients that the sweeps read eight steps later into L1: the first sweep's rows, and the
+            // first row of the others'
+            auto touch = [&](int t) {
+                const int s = image ? 0 : lane - kPipeG, i = image ? 32 * B + lane : 32 * B - s, j = t + 8 - 2 * s - (image ? lane : 0);
+                if ((image || (s > 0 && s < gs)) && i >= 0 && i < H && j >= 0 && j < W) {
+                    const double2* p = a.coef + diag_base(i + j, W, H) + i;
+#pragma unroll
+                    for (int z = 0; z < 4; z++) pipe_touch(p + (size_t)z * N);
+                }
+            };
+            auto put = [&](int t, double2 v) {
+                if (image) queue[0][(t + 1) & 3][lane] = v;
+                else if (lane <= kPipeG) edge[lane][col(t) & 3] = v;
+            };
+            for (int t = -9; t < -1; t++) touch(t);
+            // the input's row 32 B is a sweep ahead of the others: its first two columns now
+            if (!image && lane == 0)
+                for (int t = -3; t < -1; t++) put(t, wants(t) ? poll(t, pipe_load(at(t), true)) : make_double2(0, 0));
+            double2 v[kPipeAhead];
+#pragma unroll
+            for (int k = 0; k < kPipeAhead; k++) v[k] = pipe_load(at(k - 1), wants(k - 1));
+            if (__syncthreads_or(stop || gave_up)) stop = true;
+            for (int t = -1; !stop && t <= last; t += kPipeAhead) {
+#pragma unroll
+                for (int k = 0; k < kPipeAhead; k++) {
+                    if (stop || t + k > last) break;
+                    double2 x = v[k];
+                    if (wants(t + k)) x = poll(t + k, x);
+                    __syncwarp();
+                    put(t + k, x);
+                    v[k] = pipe_load(at(t + k + kPipeAhead), wants(t + k + kPipeAhead));
+                    touch(t + k);
+                    if (__syncthreads_or(stop || gave_up)) stop = true;
                 }
             }
         }
-        __syncthreads();
+        if (gave_up) {
+            atomicMin(a.conv, -1);  // every other wait stops at this too
+            *a.status = 1;
+        }
     }
-    if (threadIdx.x == 0) {
-        *sweeps = s_done + 1;
-        if (t >= t_max) *status = 1;
-    }
-    const int last = (s_stop >= 0 ? s_stop : nSOR - 1) % D;
-    for (size_t p = threadIdx.x; p < N; p += blockDim.x) {
-        const double2 x = ring[(size_t)last * N + p];
+}
+
+// The increment the sweeps end with, into (du, dv); fin: this launch group holds the last sweep.
+__global__ void k_sor_result(LevelBufs b, PipeArgs a, int fin)
+{
+    const int conv = *a.conv;
+    if (conv < a.s0 || (conv >= a.s0 + a.n && !fin)) return;
+    const int last = min(conv, a.s0 + a.n - 1), g = (last - a.s0) / a.G, ng = (a.n + a.G - 1) / a.G;
+    const bool whole = (last - a.s0) % a.G + 1 == min(a.G, a.n - g * a.G);
+    const size_t n = (size_t)b.W * b.H;
+    const double2* img = a.img + (size_t)(whole ? g + 1 : ng + 1) * n;
+    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(p / b.W), j = (int)(p % b.W);
+        const double2 x = img[diag_base(i + j, b.W, b.H) + i];
         b.du[p] = x.x;
         b.dv[p] = x.y;
     }
 }
 
-// The same SOR over a thread-block cluster of C CTAs, for the larger levels: every CTA keeps the
-// same sweep schedule (start steps, completed sweeps, the stop), decided by each CTA's thread 0
-// from the same inputs; the pixels of each step's diagonals are spread over all the cluster's
-// threads; a sweep's maximum change is the largest of the CTAs' partial maxima, read through
-// distributed shared memory.  One cluster barrier a step, after the updates (the ring's new values
-// are visible to the next step); a ring slot, with its partial-maximum slot, is reused only a step
-// after its sweep completed, so no CTA resets a partial maximum another CTA may still be reading.  The order of the updates is the single-CTA kernel's, so the
-// flow is the same bit for bit; with more sweeps in flight (D up to kMaxRingC) a step carries more
-// independent work.
-constexpr int kMaxRingC = 64;
-
-__global__ void __launch_bounds__(kSorThreads) k_sor_wavefront_cluster(LevelBufs b, double alpha, int nSOR, int D,
-                                                                       double2* ring, int* sweeps,
-                                                                       int* status)
+// Work space of a level's pipeline: how many groups of how many sweeps a launch takes within `avail` bytes.
+struct PipePlan {
+    int G, groups, NB;
+    size_t img, bnd;  // bytes of an image, of a group's last rows
+};
+static inline PipePlan pipe_plan(int W, int H, int nSOR, size_t avail)
 {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int W = b.W, H = b.H, ndiag = W + H - 1, lag = 2;
-    const size_t N = (size_t)W * H;
-    const int G = C * blockDim.x, g = rank * blockDim.x + threadIdx.x;
-    __shared__ long long start[kMaxRingC];
-    __shared__ long long fin[kMaxRingC];  // the step at which the sweep in each slot completed
-    __shared__ unsigned long long maxd[kMaxRingC];
-    __shared__ int s_done, s_stop, s_next;
-    __shared__ int pre[kMaxRingC + 1], dd[kMaxRingC], ii0[kMaxRingC];
-    if (threadIdx.x < kMaxRingC) fin[threadIdx.x] = -1;
-    for (size_t p = g; p < N; p += G) {
-        ring[(size_t)(D - 1) * N + p] = make_double2(0.0, 0.0);
+    PipePlan p{};
+    for (int G = kPipeG; G >= 1; G /= 2) {
+        p.G = G;
+        p.NB = (H + G - 1 + 31) / 32;
+        p.img = (size_t)W * H * sizeof(double2);
+        p.bnd = (size_t)p.NB * G * W * sizeof(double2);
+        const size_t fixed = 2 * p.img + p.bnd, per = p.img + p.bnd + G * sizeof(ulonglong2);
+        if (avail < fixed + per) continue;
+        p.groups = (int)std::min<size_t>((size_t)((nSOR - 1) / G + 1), (avail - fixed) / per);
+        break;
     }
-    if (threadIdx.x == 0) { s_done = -1; s_stop = -1; s_next = 0; }
-    __threadfence();
-    cl.sync();
-    const long long t_max = (long long)nSOR * (ndiag + lag) + ndiag + 8;
-    long long t = 0;
-    for (; t < t_max; t++) {
-        if (threadIdx.x < 32) {
-            // warp 0: the step's new sweep (lane 0), then the step's table.  A slot is reused one
-            // step after its sweep completed: other CTAs may read its partial maximum during the
-            // completion step, up to their next cluster barrier
-            if (threadIdx.x == 0) {
-                const int nx = s_next;
-                if (nx < nSOR && (nx == 0 || t >= start[(nx - 1) % D] + lag) &&
-                    (nx < D || (s_done >= nx - D && fin[nx % D] < t - 1))) {
-                    start[nx % D] = t;
-                    maxd[nx % D] = 0ull;
-                    s_next = nx + 1;
-                }
-            }
-            __syncwarp();
-            sor_table(W, H, t, s_done, s_next, start, D, ndiag, pre, dd, ii0);
-        }
-        __syncthreads();
-        const int done = s_done, next = s_next;
-        if (s_stop >= 0 || done >= nSOR - 1) break;  // the same in every CTA
-        sor_step<true>(b, alpha, done, next, pre, dd, ii0, D, N, ring, maxd, g, G);
-        cl.sync();  // this step's updates are done and visible in every CTA (release / acquire at cluster scope)
-        if (threadIdx.x == 0) {
-            while (s_done + 1 < s_next && t - start[(s_done + 1) % D] == ndiag - 1) {
-                s_done++;
-                fin[s_done % D] = t;
-                double mx = 0;
-                for (int r = 0; r < C; r++)
-                    mx = cmax(mx, __longlong_as_double((long long)*cl.map_shared_rank(&maxd[s_done % D], r)));
-                if (mx < 1e-5) {
-                    s_stop = s_done;
-                    break;
-                }
-            }
-        }
-    }
-    cl.sync();  // no CTA leaves while another may still read its partial maxima
-    if (rank == 0 && threadIdx.x == 0) {
-        *sweeps = s_done + 1;
-        if (t >= t_max) *status = 1;
-    }
-    const int last = (s_stop >= 0 ? s_stop : nSOR - 1) % D;
-    for (size_t p = g; p < N; p += G) {
-        const double2 x = __ldcg(ring + (size_t)last * N + p);
-        b.du[p] = x.x;
-        b.dv[p] = x.y;
-    }
+    return p;
 }
 
 // u += du, v += dv (Image::Add, SmoothFlowSOR.cpp:227-228)

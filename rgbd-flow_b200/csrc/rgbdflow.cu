@@ -768,6 +768,50 @@ static std::vector<double> gauss_taps(double sigma, int fsize)
     return g;
 }
 
+// The SOR of one inner iteration on the level `b` (k_sor_pipeline), as many sweeps a launch as the work space
+// holds; the increments are left in (b.du, b.dv).  Returns the launches.
+static int enqueue_sor_pipeline(rgbdflow_ctx* c, const rgbdflow::f2d::LevelBufs& b, double alpha, int nSOR, char* ws,
+                                size_t ws_bytes, int* ctl, cudaStream_t st)
+{
+    using namespace rgbdflow::f2d;
+    const PipePlan plan = pipe_plan(b.W, b.H, nSOR, ws_bytes);
+    if (!plan.groups) throw ArgError(RGBDFLOW_ERR_INTERNAL, "2-D SOR work space too small");
+    int launches = 0;
+    RF_CUDA(cudaMemsetAsync(ctl + 1, 0x7f, sizeof(int), st));
+    for (int s0 = 0; s0 < nSOR;) {
+        PipeArgs a{};
+        a.W = b.W;
+        a.H = b.H;
+        a.NB = plan.NB;
+        a.s0 = s0;
+        a.G = plan.G;
+        a.n = (int)std::min<long long>(nSOR - s0, (long long)plan.groups * plan.G);
+        const int ng = (a.n + a.G - 1) / a.G;
+        a.alpha = alpha;
+        a.coef = b.coef;
+        // the images, the last rows, the sweeps' records
+        const size_t img_bytes = (size_t)(ng + 2) * plan.img, bnd_bytes = (size_t)(ng + 1) * plan.bnd;
+        a.img = (double2*)ws;
+        a.bnd = (double2*)(ws + img_bytes);
+        a.sweep = (ulonglong2*)(ws + img_bytes + bnd_bytes);
+        a.conv = ctl + 1;
+        a.status = ctl;
+        a.zero_in = s0 == 0;
+        if (s0) RF_CUDA(cudaMemcpyAsync(ws, ws + (size_t)plan.groups * plan.img, plan.img, cudaMemcpyDeviceToDevice, st));
+        RF_CUDA(cudaMemsetAsync(ws + plan.img, 0xff, img_bytes - plan.img + bnd_bytes, st));
+        RF_CUDA(cudaMemsetAsync(a.sweep, 0, (size_t)a.n * sizeof(ulonglong2), st));
+        const int tasks = (int)std::min<long long>((long long)ng * plan.NB, c->sms);
+        launch_cooperative(k_sor_pipeline, tasks, kPipeThreads, st, a);
+        a.finish = 1;
+        launch_cooperative(k_sor_pipeline, std::min(plan.NB, c->sms), kPipeThreads, st, a);
+        s0 += a.n;
+        const size_t n = (size_t)b.W * b.H;
+        k_sor_result<<<(int)std::min<size_t>((n + kThreads - 1) / kThreads, (size_t)c->sms * 8), kThreads, 0, st>>>(b, a, s0 >= nSOR);
+        launches += 3;
+    }
+    return launches;
+}
+
 // The 2-D optical flow of one pair (Coarse2FineFlow, src/opticalFlowMultiscale.cpp:4-146, CELIU
 // variant, no depth maps) on the context's stream; synchronous.
 static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2, int W, int H,
@@ -839,45 +883,15 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
         o_u[i] = reserve((size_t)lev[i].w * lev[i].h * sizeof(double));
         o_v[i] = reserve((size_t)lev[i].w * lev[i].h * sizeof(double));
     }
-    const size_t o_tmpA = reserve(N0 * 3 * sizeof(double)), o_tmpB = reserve(N0 * 3 * sizeof(double));
     const size_t o_warp = reserve(N0 * 5 * sizeof(double));
     size_t o_plane[8];
     for (auto& o : o_plane) o = reserve(N0 * sizeof(double));
-    // levels of at least this many pixels run their SOR over a cluster of CTAs with more sweeps in
-    // flight (the flow does not depend on it)
-    const char* ce = std::getenv("RGBDFLOW_FLOW2D_CLUSTER_MIN_PX");
-    const long clus_min_px = ce ? std::atol(ce) : 4096L;
-    constexpr int kClusterRing = 64;
-    // the cluster: 16 CTAs where the device can co-schedule them (a non-portable size), else 8
-    static int clus_ctas = 0;
-    if (!clus_ctas) {
-        const char* cc = std::getenv("RGBDFLOW_FLOW2D_CLUSTER_CTAS");
-        int want = cc ? std::atoi(cc) : 16;
-        want = want >= 16 ? 16 : 8;
-        if (want == 16) {
-            RF_CUDA(cudaFuncSetAttribute(k_sor_wavefront_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            cudaLaunchConfig_t q = {};
-            q.gridDim = dim3(16);
-            q.blockDim = dim3(kSorThreads);
-            cudaLaunchAttribute qa[1];
-            qa[0].id = cudaLaunchAttributeClusterDimension;
-            qa[0].val.clusterDim.x = 16;
-            qa[0].val.clusterDim.y = 1;
-            qa[0].val.clusterDim.z = 1;
-            q.attrs = qa;
-            q.numAttrs = 1;
-            int nc = 0;
-            if (cudaOccupancyMaxActiveClusters(&nc, k_sor_wavefront_cluster, &q) != cudaSuccess || nc < 1) {
-                cudaGetLastError();
-                want = 8;
-            }
-        }
-        clus_ctas = want;
-    }
-    const int kClusterCtas = clus_ctas;
-    const int ring_slots = std::max(prm.sor_ring, (long)N0 >= clus_min_px ? kClusterRing : 0);
-    const size_t o_ring = reserve((size_t)ring_slots * N0 * sizeof(double2));  // (du, dv) pairs per sweep slot
     const size_t o_coef = reserve(N0 * 8 * sizeof(double));
+    // the SOR's work space; the pyramids' two temporary images, done with by then, are its first part
+    const size_t o_pipe = reserve(N0 * 6 * sizeof(double));
+    const size_t o_tmpA = o_pipe, o_tmpB = o_pipe + N0 * 3 * sizeof(double);
+    reserve((size_t)std::max(prm.sor_ring, N0 >= 4096 ? 64 : 0) * N0 * sizeof(double2));
+    const size_t pipe_bytes = total - o_pipe;
     if (c->budget && total > c->budget) throw ArgError(RGBDFLOW_ERR_BUDGET, "2-D flow needs " + std::to_string(total) + " device bytes");
     RF_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
@@ -890,7 +904,7 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
         ~Free() { if (p) { cudaFreeAsync(p, s); cudaStreamSynchronize(s); } }
     } release{base, st};
     auto D = [&](size_t o) { return (double*)(base + o); };
-    int* ctl = (int*)(base + o_ctl);
+    int* ctl = (int*)(base + o_ctl);  // status, first sweep below the threshold
     uint8_t* dbgr = (uint8_t*)(base + o_bgr);
     RF_CUDA(cudaMemcpyAsync(dbgr, bgr1, N0 * 3, cudaMemcpyHostToDevice, st));
     RF_CUDA(cudaMemcpyAsync(dbgr + N0 * 3, bgr2, N0 * 3, cudaMemcpyHostToDevice, st));
@@ -934,7 +948,7 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
         b.dy2 = D(o_plane[5]);
         b.dtdx = D(o_plane[6]);
         b.dtdy = D(o_plane[7]);
-        b.coef = D(o_coef);
+        b.coef = (double2*)(base + o_coef);
         b.W = w;
         b.H = h;
         if (k == L - 1) {
@@ -958,25 +972,7 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
             for (int hh = 0; hh < prm.n_inner; hh++) {
                 k_phi_psi<<<grid(n), kThreads, 0, st>>>(b, d5, hh == 0 ? 1 : 0, eps);
                 k_rhs<<<grid(n), kThreads, 0, st>>>(b, prm.alpha);
-                if ((long)n >= clus_min_px) {
-                    cudaLaunchConfig_t cfg = {};
-                    cfg.gridDim = dim3(kClusterCtas);
-                    cfg.blockDim = dim3(kSorThreads);
-                    cfg.stream = st;
-                    cudaLaunchAttribute at[1];
-                    at[0].id = cudaLaunchAttributeClusterDimension;
-                    at[0].val.clusterDim.x = kClusterCtas;
-                    at[0].val.clusterDim.y = 1;
-                    at[0].val.clusterDim.z = 1;
-                    cfg.attrs = at;
-                    cfg.numAttrs = 1;
-                    RF_CUDA(cudaLaunchKernelEx(&cfg, k_sor_wavefront_cluster, b, prm.alpha, nSOR, kClusterRing,
-                                               (double2*)(base + o_ring), ctl + 1, ctl));
-                } else {
-                    k_sor_wavefront<<<1, kSorThreads, 0, st>>>(b, prm.alpha, nSOR, prm.sor_ring, (double2*)(base + o_ring),
-                                                               ctl + 1, ctl);
-                }
-                launches += 3;
+                launches += 2 + enqueue_sor_pipeline(c, b, prm.alpha, nSOR, base + o_pipe, pipe_bytes, ctl, st);
             }
             k_update<<<grid(n), kThreads, 0, st>>>(b);
             k_warp<<<grid(n), kThreads, 0, st>>>(b.f1, b.f2, b.u, b.v, b.warp, w, h);
@@ -985,13 +981,13 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
     }
     RF_CUDA(cudaGetLastError());
     std::vector<double> u(N0), v(N0);
-    int hctl[2] = {0, 0};
+    int status = 0;
     RF_CUDA(cudaMemcpyAsync(u.data(), D(o_u[0]), N0 * sizeof(double), cudaMemcpyDeviceToHost, st));
     RF_CUDA(cudaMemcpyAsync(v.data(), D(o_v[0]), N0 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    RF_CUDA(cudaMemcpyAsync(hctl, ctl, sizeof(hctl), cudaMemcpyDeviceToHost, st));
+    RF_CUDA(cudaMemcpyAsync(&status, ctl, sizeof(status), cudaMemcpyDeviceToHost, st));
     RF_CUDA(cudaStreamSynchronize(st));
     c->last_launches = launches;
-    if (hctl[0]) throw ArgError(RGBDFLOW_ERR_INTERNAL, "2-D SOR ran out of its step bound");
+    if (status) throw ArgError(RGBDFLOW_ERR_INTERNAL, "2-D SOR ran out of its step bound");
     for (size_t z = 0; z < N0; z++) {
         flow_out[z * 2] = (float)u[z];
         flow_out[z * 2 + 1] = (float)v[z];

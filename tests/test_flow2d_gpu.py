@@ -79,3 +79,36 @@ def test_cluster_sor_equals_single_cta_on_a_config_pair(ctx, monkeypatch):
     monkeypatch.setenv("RGBDFLOW_FLOW2D_CLUSTER_MIN_PX", "1")
     b = ctx.optical_flow_2d(p["bgr1"], p["bgr2"])
     np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("w, h, n_sor, over", [
+    (37, 29, 1, {}), (33, 32, 7, {}), (31, 33, 8, {}), (65, 70, 9, {}), (3, 97, 21, dict(min_width=3)),
+    (100, 5, 40, dict(min_width=60)), (2, 2, 5, dict(min_width=2)),
+    (37, 29, 100, dict(sor_ring=2)),    # work space for one group of sweeps a launch
+    (40, 40, 400, dict(alpha=0.5)),
+], ids=str)
+def test_sor_pipeline_equals_oracle_at_its_edges(ctx, w, h, n_sor, over):
+    """Widths and heights around a band's 32 rows, sweep counts around a group's 8, several launches a solve:
+    the arithmetic and its order are the oracle's, so the flow is equal."""
+    rng = np.random.default_rng(w * 1000 + h)
+    b1 = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+    b2 = np.clip(np.roll(b1, 1, axis=1).astype(int) + rng.integers(-3, 4, b1.shape), 0, 255).astype(np.uint8)
+    q = dict(dict(min_width=20, n_outer=2, n_inner=2), **over)
+    flow = ctx.optical_flow_2d(b1, b2, rf.flow2d_params(n_sor=n_sor, **q))
+    q.pop("sor_ring", None)
+    u, v = ob.optical_flow_2d(b1, b2, n_sor=n_sor, **q)
+    np.testing.assert_array_equal(flow, np.stack([u, v], -1).astype(np.float32))
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_sor_pipeline_stops_at_the_first_converged_sweep(ctx, seed):
+    """Frames that are equal (the first sweep converges) in all but a faint patch, whose sweeps converge inside a
+    group: the increments are that sweep's."""
+    rng = np.random.default_rng(seed)
+    b1 = np.full((48, 60, 3), 90, np.uint8)
+    b2 = b1.copy()
+    b1[10 * seed:10 * seed + 6, 20:30] += rng.integers(0, 3, (6, 10, 3), dtype=np.uint8)
+    for n_sor in (3, 400):
+        flow = ctx.optical_flow_2d(b1, b2, rf.flow2d_params(n_sor=n_sor, n_outer=2))
+        u, v = ob.optical_flow_2d(b1, b2, n_sor=n_sor, n_outer=2)
+        np.testing.assert_array_equal(flow, np.stack([u, v], -1).astype(np.float32))
