@@ -127,8 +127,9 @@ template <> __device__ __forceinline__ float tof<float>(float v) { return v; }
 template <> __device__ __forceinline__ float tof<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float tof<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-template <class T, class S> __device__ __forceinline__ T ldS(const S* p) { return (T)tof<S>(p[0]); }
-template <> __device__ __forceinline__ double ldS<double, double>(const double* p) { return p[0]; }
+// A feature or depth plane's value; the planes do not change while a level is solved.
+template <class T, class S> __device__ __forceinline__ T ldS(const S* p) { return (T)tof<S>(__ldg(p)); }
+template <> __device__ __forceinline__ double ldS<double, double>(const double* p) { return __ldg(p); }
 
 template <class S> __device__ __forceinline__ S fromT(float v);
 template <> __device__ __forceinline__ float fromT<float>(float v) { return v; }
@@ -652,6 +653,160 @@ __global__ void k_level_setup(const LevelItem<T, S>* items, const Tile* tiles, i
 constexpr int LRW = LTW + 4, LRH = LTH + 4;  // warped region (halo 2)
 template <class T> constexpr size_t lin_smem_bytes() { return sizeof(T) * 19 * LRW * LRH; }
 
+// The shared planes of a linearisation over a window of the image: plane p's value of pixel (i, j).
+template <class T, int PITCH>
+struct LinPlanes {
+    T* base;
+    int y, x;       // pixel of the window's first element
+    int pitch, n;   // elements of a row, of a plane (PITCH > 0: a constant window of LRH rows)
+    __device__ __forceinline__ T& at(int p, int i, int j) const
+    {
+        return PITCH > 0 ? base[p * (PITCH * LRH) + (i - y) * PITCH + (j - x)] : base[p * n + (i - y) * pitch + (j - x)];
+    }
+};
+// [6] 0.4*I1 + 0.6*warped I2 (5 features + depth), [6] warped I2 - I1, [3] flow u, [3] u + du, robust smoothness weight
+constexpr int kLinB = 0, kLinDT = 6, kLinU = 12, kLinUD = 15, kLinPhi = 18, kLinN = 19;
+
+// Warps frame 2 to pixel (gi, gj) by its flow U: planes B and DT.
+template <class T, class S, class V>
+__device__ __forceinline__ void lin_warp_px(const LevelItem<T, S>& it, const V& sv, int gi, int gj, const T* U)
+{
+    const int W = it.W, H = it.H, l = gi * W + gj;
+    const T x = (T)gj + U[0], y = (T)gi + U[1];
+    T wI[6], I1v[6];
+    for (int c = 0; c < 5; c++) I1v[c] = ldS<T, S>(it.I1[c] + l);
+    I1v[5] = ldS<T, S>(it.D1 + l);
+    if (x < 0 || x > (T)(W - 1) || y < 0 || y > (T)(H - 1)) {
+        for (int c = 0; c < 5; c++) wI[c] = I1v[c];
+        wI[5] = I1v[5] - U[2];
+    } else {
+        const int xa = clampi((int)floor(x), 0, W - 1), ya = clampi((int)floor(y), 0, H - 1);
+        const int xb = min(W - 1, xa + 1), yb = min(H - 1, ya + 1);
+        const T ax = x - (T)xa, ay = y - (T)ya;
+        const T w00 = (1 - ax) * (1 - ay), w01 = (1 - ax) * ay, w10 = ax * (1 - ay), w11 = ax * ay;
+        const int p00 = ya * W + xa, p01 = yb * W + xa, p10 = ya * W + xb, p11 = yb * W + xb;
+        for (int c = 0; c < 5; c++) {
+            const S* s = it.I2[c];
+            wI[c] = w00 * ldS<T, S>(s + p00) + w01 * ldS<T, S>(s + p01) + w10 * ldS<T, S>(s + p10) +
+                    w11 * ldS<T, S>(s + p11);
+        }
+        const S* s = it.D2;
+        wI[5] = w00 * ldS<T, S>(s + p00) + w01 * ldS<T, S>(s + p01) + w10 * ldS<T, S>(s + p10) +
+                w11 * ldS<T, S>(s + p11) - U[2];
+    }
+    for (int c = 0; c < 6; c++) {
+        sv.at(kLinB + c, gi, gj) = (T).4 * I1v[c] + (T).6 * wI[c];
+        sv.at(kLinDT + c, gi, gj) = wI[c] - I1v[c];
+    }
+}
+
+// The robust smoothness weight phi of pixel (gi, gj).
+template <class T, class S, class V>
+__device__ __forceinline__ void lin_phi_px(const LevelItem<T, S>& it, const SolveConst<T>& k, const V& sv, int gi, int gj)
+{
+    T d[6];
+    for (int c = 0; c < 3; c++) {
+        d[2 * c] = (gj == it.W - 1) ? (T)0 : sv.at(kLinUD + c, gi, gj + 1) - sv.at(kLinUD + c, gi, gj);
+        d[2 * c + 1] = (gi == it.H - 1) ? (T)0 : sv.at(kLinUD + c, gi + 1, gj) - sv.at(kLinUD + c, gi, gj);
+    }
+    const T s = __ldg(it.pyr[9] + gi * it.W + gj);
+    const T q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3] + s * (d[4] * d[4] + d[5] * d[5]);
+    sv.at(kLinPhi, gi, gj) = (T)0.5 * rsqrtT<T>(q + k.eps_s);
+}
+
+// The system of pixel (gi, gj): o[0..11] (the sys planes), and of its left and upper edge the weight (sys[9] /
+// sys[10] of the pixel there) and that pixel's depth-smoothness weight: e[0..3].
+template <class T, class S, class V>
+__device__ __forceinline__ void lin_system_px(const LevelItem<T, S>& it, const SolveConst<T>& k, const V& sv, int gi, int gj,
+                                              T* o, T* edge)
+{
+    const int W = it.W, H = it.H, l = gi * W + gj;
+    const T gfl[5] = {1, -8, 0, 8, -1};
+    T Ix[6], Iy[6], It[6];
+    for (int c = 0; c < 6; c++) {
+        T sx = 0, sy = 0;
+        for (int m = 0; m < 5; m++) {
+            const int cc = clampi(gj - 2 + m, 0, W - 1);
+            const int rr = clampi(gi - 2 + m, 0, H - 1);
+            sx += gfl[m] * sv.at(kLinB + c, gi, cc);
+            sy += gfl[m] * sv.at(kLinB + c, rr, gj);
+        }
+        Ix[c] = sx / (T)12;
+        Iy[c] = sy / (T)12;
+        It[c] = sv.at(kLinDT + c, gi, gj);
+    }
+    Ix[5] = minT(maxT(Ix[5], -k.max_grad), k.max_grad);
+    Iy[5] = minT(maxT(Iy[5], -k.max_grad), k.max_grad);
+    It[5] = minT(maxT(It[5], -k.max_grad), k.max_grad);
+    const T U0 = sv.at(kLinU, gi, gj), U1 = sv.at(kLinU + 1, gi, gj), U2 = sv.at(kLinU + 2, gi, gj);
+    const T du0 = sv.at(kLinUD, gi, gj) - U0, du1 = sv.at(kLinUD + 1, gi, gj) - U1, du2 = sv.at(kLinUD + 2, gi, gj) - U2;
+    const T z1 = ldS<T, S>(it.D1 + l);
+    const T q = (z1 + U2 < ldS<T, S>(it.D2 + l) + k.occ_margin * (z1 * z1)) ? (T)1 : k.occ_penalty;
+    T sxy = 0, sx2 = 0, sy2 = 0, stx = 0, sty = 0;
+    for (int c = 0; c < 5; c++) {
+        const T e = (It[c] + Ix[c] * du0 + Iy[c] * du1) * q;
+        const T psi = (T)0.5 * rsqrtT<T>(e * e + k.eps_d) * k.color_w;
+        sxy += psi * Ix[c] * Iy[c];
+        sx2 += psi * Ix[c] * Ix[c];
+        sy2 += psi * Iy[c] * Iy[c];
+        stx += psi * Ix[c] * It[c];
+        sty += psi * Iy[c] * It[c];
+    }
+    const T ixy = sxy / (T)5, ix2 = sx2 / (T)5, iy2 = sy2 / (T)5;
+    const T itx = stx * q * q / (T)5, ity = sty * q * q / (T)5;
+    const T e2 = It[5] + Ix[5] * du0 + Iy[5] * du1 - du2;
+    const T pi = (T)0.5 * rsqrtT<T>(e2 * e2 + k.eps_z) * __ldg(it.pyr[8] + l);
+    const T dxy = pi * Ix[5] * Iy[5], dx2 = pi * Ix[5] * Ix[5], dy2 = pi * Iy[5] * Iy[5];
+    const T dtx = pi * Ix[5] * It[5], dty = pi * Iy[5] * It[5];
+    // weighted Laplacians of u (not u + du) and edge weights
+    const bool hasR = gj < W - 1, hasL = gj > 0, hasD = gi < H - 1, hasU = gi > 0;
+    const T rhl = __ldg(it.rh + l), rvl = __ldg(it.rv + l);
+    const T rhL = hasL ? __ldg(it.rh + l - 1) : (T)0, rvU = hasU ? __ldg(it.rv + l - W) : (T)0;
+    const T phi = sv.at(kLinPhi, gi, gj);
+    const T phiL = hasL ? sv.at(kLinPhi, gi, gj - 1) : (T)0, phiU = hasU ? sv.at(kLinPhi, gi - 1, gj) : (T)0;
+    T nrm = 0;
+    int cnt = 0;
+    if (hasR) { nrm += rhl; cnt++; }
+    if (hasL) { nrm += rhL; cnt++; }
+    if (hasD) { nrm += rvl; cnt++; }
+    if (hasU) { nrm += rvU; cnt++; }
+    T lap[3];
+    for (int c = 0; c < 3; c++) {
+        T lv = 0;
+        const T uc = sv.at(kLinU + c, gi, gj);
+        if (hasR) lv -= (sv.at(kLinU + c, gi, gj + 1) - uc) * phi * rhl;
+        if (hasL) lv += (uc - sv.at(kLinU + c, gi, gj - 1)) * phiL * rhL;
+        if (hasD) lv -= (sv.at(kLinU + c, gi + 1, gj) - uc) * phi * rvl;
+        if (hasU) lv += (uc - sv.at(kLinU + c, gi - 1, gj)) * phiU * rvU;
+        lap[c] = (absT(nrm) < (T)1e-5) ? (T)0 : lv / (nrm / (T)cnt);
+    }
+    const T s = __ldg(it.pyr[9] + l);
+    const T sL = hasL ? __ldg(it.pyr[9] + l - 1) : (T)0, sU_ = hasU ? __ldg(it.pyr[9] + l - W) : (T)0;
+    T sumXY = 0, sumZ = 0;
+    if (hasL) { const T e = phiL * rhL; sumXY += e; sumZ += e * sL; }
+    if (hasU) { const T e = phiU * rvU; sumXY += e; sumZ += e * sU_; }
+    if (hasR) { const T e = phi * rhl; sumXY += e; sumZ += e * s; }
+    if (hasD) { const T e = phi * rvl; sumXY += e; sumZ += e * s; }
+    const T al = k.alpha, ga = k.gamma, mg = __ldg(it.mag + l);
+    // reciprocals of the diagonal: the SOR multiplies instead of dividing
+    o[0] = (T)1 / (-(ix2 + dx2 + al * sumXY) - ga);
+    o[1] = (T)1 / (-(iy2 + dy2 + al * sumXY) - ga);
+    o[2] = (T)1 / (-(pi + al * sumZ) - ga * mg);
+    o[3] = -ixy - dxy;
+    o[4] = pi * Ix[5];
+    o[5] = pi * Iy[5];
+    o[6] = -(-itx - dtx + al * -lap[0]) + ga * U0;
+    o[7] = -(-ity - dty + al * -lap[1]) + ga * U1;
+    o[8] = -(pi * It[5] + al * -(s * lap[2])) + ga * mg * U2;
+    o[9] = hasR ? al * (phi * rhl) : (T)0;
+    o[10] = hasD ? al * (phi * rvl) : (T)0;
+    o[11] = s;
+    edge[0] = hasL ? al * (phiL * rhL) : (T)0;
+    edge[1] = hasU ? al * (phiU * rvU) : (T)0;
+    edge[2] = sL;
+    edge[3] = sU_;
+}
+
 template <class T, class S>
 __global__ void __launch_bounds__(LTW * LTH)
 k_linearize(const LevelItem<T, S>* items, const Tile* tiles, SolveConst<T> k, int use_du, int xsel)
@@ -674,161 +829,40 @@ k_linearize(const LevelItem<T, S>* items, const Tile* tiles, SolveConst<T> k, in
     // the increment of the inner iteration before: planes xsel, or (< 0) where the register kernels left it
     const int xb = use_du ? (xsel < 0 ? ctl->x_stop : xsel) : 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    typedef T Plane[LRH][LRW];
-    Plane* sB = reinterpret_cast<Plane*>(smem_raw);  // [6] 0.4*I1 + 0.6*warped I2 (5 features + depth)
-    Plane* sDT = sB + 6;                              // [6] warped I2 - I1
-    Plane* sU = sDT + 6;                              // [3] flow u
-    Plane* sUD = sU + 3;                              // [3] u + du
-    Plane& sPhi = *(sUD + 3);                         // robust smoothness weight
+    const LinPlanes<T, LRW> sv{reinterpret_cast<T*>(smem_raw), y0 - 2, x0 - 2, LRW, LRW * LRH};
     const int tid = threadIdx.x;
     for (int r = tid; r < LRW * LRH; r += blockDim.x) {
-        const int ry = r / LRW, rx = r % LRW;
-        const int gi = y0 - 2 + ry, gj = x0 - 2 + rx;
+        const int gi = y0 - 2 + r / LRW, gj = x0 - 2 + r % LRW;
         if (gi < 0 || gj < 0 || gi >= H || gj >= W) continue;
-        const int l = gi * W + gj, lp = gi * it.pitch + gj;
+        const int lp = gi * it.pitch + gj;
         T U[3], D[3];
         for (int c = 0; c < 3; c++) {
             U[c] = it.u[c][lp];
             D[c] = use_du ? it.x[xb][c][cs_idx(gi, gj, it.hwp)] : (T)0;
-            sU[c][ry][rx] = U[c];
-            sUD[c][ry][rx] = U[c] + D[c];
+            sv.at(kLinU + c, gi, gj) = U[c];
+            sv.at(kLinUD + c, gi, gj) = U[c] + D[c];
         }
-        const T x = (T)gj + U[0], y = (T)gi + U[1];
-        T wI[6], I1v[6];
-        for (int c = 0; c < 5; c++) I1v[c] = ldS<T, S>(it.I1[c] + l);
-        I1v[5] = ldS<T, S>(it.D1 + l);
-        if (x < 0 || x > (T)(W - 1) || y < 0 || y > (T)(H - 1)) {
-            for (int c = 0; c < 5; c++) wI[c] = I1v[c];
-            wI[5] = I1v[5] - U[2];
-        } else {
-            const int xa = clampi((int)floor(x), 0, W - 1), ya = clampi((int)floor(y), 0, H - 1);
-            const int xb = min(W - 1, xa + 1), yb = min(H - 1, ya + 1);
-            const T ax = x - (T)xa, ay = y - (T)ya;
-            const T w00 = (1 - ax) * (1 - ay), w01 = (1 - ax) * ay, w10 = ax * (1 - ay), w11 = ax * ay;
-            const int p00 = ya * W + xa, p01 = yb * W + xa, p10 = ya * W + xb, p11 = yb * W + xb;
-            for (int c = 0; c < 5; c++) {
-                const S* s = it.I2[c];
-                wI[c] = w00 * ldS<T, S>(s + p00) + w01 * ldS<T, S>(s + p01) + w10 * ldS<T, S>(s + p10) +
-                        w11 * ldS<T, S>(s + p11);
-            }
-            const S* s = it.D2;
-            wI[5] = w00 * ldS<T, S>(s + p00) + w01 * ldS<T, S>(s + p01) + w10 * ldS<T, S>(s + p10) +
-                    w11 * ldS<T, S>(s + p11) - U[2];
-        }
-        for (int c = 0; c < 6; c++) {
-            sB[c][ry][rx] = (T).4 * I1v[c] + (T).6 * wI[c];
-            sDT[c][ry][rx] = wI[c] - I1v[c];
-        }
+        lin_warp_px<T, S>(it, sv, gi, gj, U);
     }
     __syncthreads();
     // robust smoothness weight phi on the interior plus the column to its left and the row above
     for (int r = tid; r < (LTW + 1) * (LTH + 1); r += blockDim.x) {
-        const int ry = 1 + r / (LTW + 1), rx = 1 + r % (LTW + 1);
-        const int gi = y0 - 2 + ry, gj = x0 - 2 + rx;
+        const int gi = y0 - 1 + r / (LTW + 1), gj = x0 - 1 + r % (LTW + 1);
         if (gi < 0 || gj < 0 || gi >= H || gj >= W) continue;
-        T d[6];
-        for (int c = 0; c < 3; c++) {
-            d[2 * c] = (gj == W - 1) ? (T)0 : sUD[c][ry][rx + 1] - sUD[c][ry][rx];
-            d[2 * c + 1] = (gi == H - 1) ? (T)0 : sUD[c][ry + 1][rx] - sUD[c][ry][rx];
-        }
-        const T s = it.pyr[9][gi * W + gj];
-        const T q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3] + s * (d[4] * d[4] + d[5] * d[5]);
-        sPhi[ry][rx] = (T)0.5 * rsqrtT<T>(q + k.eps_s);
+        lin_phi_px<T, S>(it, k, sv, gi, gj);
     }
     __syncthreads();
-    const int lx = tid % LTW, ly = tid / LTW;
-    const int gi = y0 + ly, gj = x0 + lx;
+    const int gi = y0 + tid / LTW, gj = x0 + tid % LTW;
+    const int lp = cs_idx(gi, gj, it.hwp);
     if (gi < H && gj >= W && gj < 2 * it.hwp) {
         // the half-rows' padding: the register SOR reads whole half-rows, and a pixel outside the image has
         // a system of zeros
-        const int lp = cs_idx(gi, gj, it.hwp);
         for (int c = 0; c < 12; c++) it.sys[c][lp] = (T)0;
     }
     if (gi >= H || gj >= W) return;
-    const int l = gi * W + gj;
-    const int ry = ly + 2, rx = lx + 2;
-    const T gfl[5] = {1, -8, 0, 8, -1};
-    T Ix[6], Iy[6], It[6];
-    for (int c = 0; c < 6; c++) {
-        T sx = 0, sy = 0;
-        for (int m = 0; m < 5; m++) {
-            const int cc = clampi(gj - 2 + m, 0, W - 1) - (x0 - 2);
-            const int rr = clampi(gi - 2 + m, 0, H - 1) - (y0 - 2);
-            sx += gfl[m] * sB[c][ry][cc];
-            sy += gfl[m] * sB[c][rr][rx];
-        }
-        Ix[c] = sx / (T)12;
-        Iy[c] = sy / (T)12;
-        It[c] = sDT[c][ry][rx];
-    }
-    Ix[5] = minT(maxT(Ix[5], -k.max_grad), k.max_grad);
-    Iy[5] = minT(maxT(Iy[5], -k.max_grad), k.max_grad);
-    It[5] = minT(maxT(It[5], -k.max_grad), k.max_grad);
-    const T U0 = sU[0][ry][rx], U1 = sU[1][ry][rx], U2 = sU[2][ry][rx];
-    const T du0 = sUD[0][ry][rx] - U0, du1 = sUD[1][ry][rx] - U1, du2 = sUD[2][ry][rx] - U2;
-    const T z1 = ldS<T, S>(it.D1 + l);
-    const T q = (z1 + U2 < ldS<T, S>(it.D2 + l) + k.occ_margin * (z1 * z1)) ? (T)1 : k.occ_penalty;
-    T sxy = 0, sx2 = 0, sy2 = 0, stx = 0, sty = 0;
-    for (int c = 0; c < 5; c++) {
-        const T e = (It[c] + Ix[c] * du0 + Iy[c] * du1) * q;
-        const T psi = (T)0.5 * rsqrtT<T>(e * e + k.eps_d) * k.color_w;
-        sxy += psi * Ix[c] * Iy[c];
-        sx2 += psi * Ix[c] * Ix[c];
-        sy2 += psi * Iy[c] * Iy[c];
-        stx += psi * Ix[c] * It[c];
-        sty += psi * Iy[c] * It[c];
-    }
-    const T ixy = sxy / (T)5, ix2 = sx2 / (T)5, iy2 = sy2 / (T)5;
-    const T itx = stx * q * q / (T)5, ity = sty * q * q / (T)5;
-    const T e2 = It[5] + Ix[5] * du0 + Iy[5] * du1 - du2;
-    const T pi = (T)0.5 * rsqrtT<T>(e2 * e2 + k.eps_z) * it.pyr[8][l];
-    const T dxy = pi * Ix[5] * Iy[5], dx2 = pi * Ix[5] * Ix[5], dy2 = pi * Iy[5] * Iy[5];
-    const T dtx = pi * Ix[5] * It[5], dty = pi * Iy[5] * It[5];
-    // weighted Laplacians of u (not u + du) and edge weights
-    const bool hasR = gj < W - 1, hasL = gj > 0, hasD = gi < H - 1, hasU = gi > 0;
-    const T rhl = it.rh[l], rvl = it.rv[l];
-    const T rhL = hasL ? it.rh[l - 1] : (T)0, rvU = hasU ? it.rv[l - W] : (T)0;
-    const T phi = sPhi[ry][rx];
-    const T phiL = hasL ? sPhi[ry][rx - 1] : (T)0, phiU = hasU ? sPhi[ry - 1][rx] : (T)0;
-    T nrm = 0;
-    int cnt = 0;
-    if (hasR) { nrm += rhl; cnt++; }
-    if (hasL) { nrm += rhL; cnt++; }
-    if (hasD) { nrm += rvl; cnt++; }
-    if (hasU) { nrm += rvU; cnt++; }
-    T lap[3];
-    for (int c = 0; c < 3; c++) {
-        T lv = 0;
-        const T uc = sU[c][ry][rx];
-        if (hasR) lv -= (sU[c][ry][rx + 1] - uc) * phi * rhl;
-        if (hasL) lv += (uc - sU[c][ry][rx - 1]) * phiL * rhL;
-        if (hasD) lv -= (sU[c][ry + 1][rx] - uc) * phi * rvl;
-        if (hasU) lv += (uc - sU[c][ry - 1][rx]) * phiU * rvU;
-        lap[c] = (absT(nrm) < (T)1e-5) ? (T)0 : lv / (nrm / (T)cnt);
-    }
-    const T s = it.pyr[9][l];
-    const T sL = hasL ? it.pyr[9][l - 1] : (T)0, sU_ = hasU ? it.pyr[9][l - W] : (T)0;
-    T sumXY = 0, sumZ = 0;
-    if (hasL) { const T e = phiL * rhL; sumXY += e; sumZ += e * sL; }
-    if (hasU) { const T e = phiU * rvU; sumXY += e; sumZ += e * sU_; }
-    if (hasR) { const T e = phi * rhl; sumXY += e; sumZ += e * s; }
-    if (hasD) { const T e = phi * rvl; sumXY += e; sumZ += e * s; }
-    const T al = k.alpha, ga = k.gamma, mg = it.mag[l];
-    T* const* o = it.sys;
-    const int lp = cs_idx(gi, gj, it.hwp);
-    // reciprocals of the diagonal: the SOR multiplies instead of dividing
-    o[0][lp] = (T)1 / (-(ix2 + dx2 + al * sumXY) - ga);
-    o[1][lp] = (T)1 / (-(iy2 + dy2 + al * sumXY) - ga);
-    o[2][lp] = (T)1 / (-(pi + al * sumZ) - ga * mg);
-    o[3][lp] = -ixy - dxy;
-    o[4][lp] = pi * Ix[5];
-    o[5][lp] = pi * Iy[5];
-    o[6][lp] = -(-itx - dtx + al * -lap[0]) + ga * U0;
-    o[7][lp] = -(-ity - dty + al * -lap[1]) + ga * U1;
-    o[8][lp] = -(pi * It[5] + al * -(s * lap[2])) + ga * mg * U2;
-    o[9][lp] = hasR ? al * (phi * rhl) : (T)0;
-    o[10][lp] = hasD ? al * (phi * rvl) : (T)0;
-    o[11][lp] = s;
+    T o[12], edge[4];
+    lin_system_px<T, S>(it, k, sv, gi, gj, o, edge);
+    for (int c = 0; c < 12; c++) it.sys[c][lp] = o[c];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2228,8 +2262,28 @@ k_sor_level_cluster_reg(const LevelItem<T, S>* items, const int* which, SolveCon
 
 // After each outer iteration: the early-termination statistic of the pair (mean over 3N of
 // sqr(du) * (1, 1, f / depth1), .cu:943-951), the stop decision and the executed-schedule record.
-// One warp per item (lane = the thread's lane); the statistic partials are read from L2 (the
-// whole-level cluster kernel calls this after other CTAs wrote them).
+// One warp per item (lane = the thread's lane); the statistic partials are read from L2 (other CTAs may have
+// written them).
+template <class T, class S>
+__device__ __forceinline__ bool control_decide(const LevelItem<T, S>& it, const SolveConst<T>& k, T stat)
+{
+    return it.allow_early && !k.fixed && (double)stat / ((double)it.W * it.H * 3) < k.outer_tol;
+}
+// stat: the statistic's sum; iters: SOR iterations executed; maxdiff: the last convergence check's change (-1: none).
+template <class T, class S>
+__device__ __forceinline__ void control_record(const LevelItem<T, S>& it, const SolveConst<T>& k, int outer, T stat, int iters,
+                                               float maxdiff, bool done)
+{
+    PairCtl* ctl = it.ctl;
+    const int lv = it.level;
+    if (outer < 64) {
+        ctl->sor_exec[lv][outer] = iters;
+        ctl->stat[lv][outer] = (it.allow_early && !k.fixed) ? (float)((double)stat / ((double)it.W * it.H * 3)) : -1.0f;
+        ctl->sor_maxdiff[lv][outer] = maxdiff;
+    }
+    ctl->outer_exec[lv] = outer + 1;
+    if (done) ctl->level_done = 1;
+}
 template <class T, class S>
 __device__ __forceinline__ void control_item(const LevelItem<T, S>& it, const SolveConst<T>& k, int outer, int n_checks,
                                              int lane)
@@ -2240,20 +2294,16 @@ __device__ __forceinline__ void control_item(const LevelItem<T, S>& it, const So
     for (int i = lane; i < it.n_sor_tiles; i += 32) s += __ldcg(it.stat_part + i);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) {
-        const double st = (double)s / ((double)it.W * it.H * 3);
-        const int lv = it.level;
-        if (outer < 64) {
-            ctl->sor_exec[lv][outer] = ctl->sor_stop ? ctl->sor_stop_iter : k.n_sor;
-            ctl->stat[lv][outer] = (it.allow_early && !k.fixed) ? (float)st : -1.0f;
-            float md = -1.0f;  // the last convergence check evaluated in this outer iteration
-            for (int c = min(n_checks, kMaxChecks) - 1; c >= 0; c--) {
-                const unsigned b = ctl->maxdiff[c];
-                if (b) { md = __uint_as_float(b); break; }
-            }
-            ctl->sor_maxdiff[lv][outer] = md;
+        const int stop = ctl->sor_stop;
+        // the last convergence check evaluated in this outer iteration that saw a change (none later than the stop)
+        int c = min(n_checks, kMaxChecks) - 1;
+        if (stop) c = min(c, ctl->sor_stop_iter / k.period - 1);
+        float md = -1.0f;
+        for (; c >= 0; c--) {
+            const unsigned b = ctl->maxdiff[c];
+            if (b) { md = __uint_as_float(b); break; }
         }
-        ctl->outer_exec[lv] = outer + 1;
-        if (it.allow_early && !k.fixed && st < k.outer_tol) ctl->level_done = 1;
+        control_record(it, k, outer, s, stop ? ctl->sor_stop_iter : k.n_sor, md, control_decide(it, k, s));
     }
 }
 

@@ -21,6 +21,7 @@
 #include "kernels.cuh"
 #include "hpb.cuh"
 #include "sor_regs.cuh"
+#include "level_bands.cuh"
 
 namespace rgbdflow {
 
@@ -193,6 +194,7 @@ struct SorChoice {
     int seg = 0;     // strip band height (0: automatic)
     BandMap bands;   // explicit band layouts (strip_balanced_bands); strips of other heights use seg
     int res_k = 0;         // resident SOR from registers, this many iterations between exchanges
+    int band_c = 0;        // the level in one launch, this many CTAs an item
     double us_per_it = 0;  // measured time per SOR iteration of the step
 };
 struct TuneTable {
@@ -249,6 +251,30 @@ static inline int resident_fit(int W, int H, int kmax, int ctas)
     for (int K = kmax; K >= 1; K--)
         if (res_tiles(W, kResCols, K) * res_tiles(H, kResRows, K) <= ctas) return K;
     return 0;
+}
+
+// CTAs per item for k_level_bands on a step of n items, 0: not on it.  All clusters have to run together
+// (clusters of 16, 8, 4, 2 CTAs, one CTA an SM, of which the device holds 7, 16, 35, 74 at once), and a
+// band has to fit a CTA.  Among those the cheapest half-sweep: an update takes a scheduler 105 cycles a warp, its
+// chain about 200, a cluster barrier 330 more than a block's.
+template <class X>
+static int band_ctas(const std::vector<X>& items, int sms)
+{
+    static const int sizes[5][2] = {{16, 7}, {8, 16}, {4, 35}, {2, 74}, {1, 148}};
+    int best = 0, best_cost = 1 << 30;
+    for (const auto& q : sizes) {
+        const int C = q[0];
+        bool fits = (int)items.size() <= q[1] && (int)items.size() * C <= sms;
+        int most = 0;
+        for (const auto& x : items) {
+            const int P = band_rows(x.H, C) * ((x.W + 1) / 2);
+            fits = fits && P <= kBandMax && (C == 1 || x.H >= 2 * C) && band_smem_bytes(x.W, x.H, C) <= kBandSmem;
+            most = std::max(most, P);
+        }
+        const int cost = 105 * ((most + 127) / 128) + (C > 1 ? 330 : 0);
+        if (fits && cost < best_cost) { best = C; best_cost = cost; }
+    }
+    return best;
 }
 
 // Iterations between the exchanges of the resident SOR, for the items of one step: a larger K exchanges less
@@ -543,6 +569,8 @@ struct Plan {
         int res_k, res_tiles;                 // iterations between exchanges, tiles of the step
         int n_fold;                           // blocks of its fold (32 x 32 tiles)
         bool regs;                            // the step's items all run from registers
+        int band_c, band_threads;             // > 0: the step runs on k_level_bands, band_c CTAs an item
+        size_t band_smem;
     };
     std::vector<StepDesc> steps;
     struct PyrLevelDesc { size_t jobs_off; int n_jobs; size_t src_tiles_off; int n_src; size_t dst_tiles_off; int n_dst; size_t g_off; };
@@ -979,9 +1007,17 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         P.step_tuned.push_back(ch != nullptr);
         const bool strips = ch ? ch->strip != 0 : strip_px >= (hp.strip_min_px > 0 ? hp.strip_min_px : 2000000L);
         std::vector<int> res_items;
+        const int band_c = regs && hp.res_k == 0 ? band_ctas(items, ctas) : 0;
+        int band_thr = 256;
+        size_t band_smem = 0;
         for (auto& x : items) {
             const int sx = (x.W + kSorTW - 1) / kSorTW, sy = (x.H + kSorTH - 1) / kSorTH;
             x.n_sor_tiles = sx * sy;
+            if (band_c) {
+                band_thr = std::max(band_thr, (band_rows(x.H, band_c) * ((x.W + 1) / 2) + 31) / 32 * 32);
+                band_smem = std::max(band_smem, band_smem_bytes(x.W, x.H, band_c));
+                continue;
+            }
             if (regs) {
                 const int i = (int)(&x - items.data());
                 if (whole_ok(x.H, x.hwp)) {
@@ -1069,6 +1105,9 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
                          [&](int a, int b) { return (long)items[a].W * items[a].H > (long)items[b].W * items[b].H; });
         std::vector<ResItem> ri;
         d.regs = regs;
+        d.band_c = band_c;
+        d.band_threads = band_thr;
+        d.band_smem = band_smem;
         d.res_k = 0;
         d.res_tiles = 0;
         d.n_fold = 0;
@@ -1386,6 +1425,11 @@ static void set_kernel_attrs()
     RF_CUDA(cudaFuncSetAttribute(k_sor_level<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemMax));
     RF_CUDA(cudaFuncSetAttribute(k_sor_level_cluster<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemMax));
     if constexpr (sizeof(T) == 4) {
+        for (auto* kernel : {k_level_bands<S, kBandSmall, true>, k_level_bands<S, kBandMax, true>,
+                             k_level_bands<S, kBandSmall, false>, k_level_bands<S, kBandMax, false>}) {
+            RF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBandSmem));
+            RF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        }
         RF_CUDA(cudaFuncSetAttribute(k_sor_level_reg<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         RF_CUDA(cudaFuncSetAttribute(k_sor_level_cluster_reg<T, S, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         RF_CUDA(cudaFuncSetAttribute(k_sor_level_cluster_reg<T, S, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
@@ -1488,6 +1532,28 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
         RF_PROF_E(pf, st);
         launches++;
     }
+    if constexpr (sizeof(T) == 4)
+        if (d.band_c) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(d.n_items * d.band_c);
+            cfg.blockDim = dim3(d.band_threads);
+            cfg.dynamicSmemBytes = d.band_smem;
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = d.band_c;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            RF_PROF_B(pf, KC_SOR_LEVEL0 + P.Lmax - 1 - sidx, st);
+            const bool small = d.band_threads <= kBandSmall;
+            auto* const kernel = d.band_c > 1 ? (small ? k_level_bands<S, kBandSmall, true> : k_level_bands<S, kBandMax, true>)
+                                              : (small ? k_level_bands<S, kBandSmall, false> : k_level_bands<S, kBandMax, false>);
+            RF_CUDA(cudaLaunchKernelEx(&cfg, kernel, items, k, d.band_c, P.hp.n_outer, P.hp.n_inner, P.status));
+            RF_PROF_E(pf, st);
+            return launches + 1;
+        }
     // a step whose items are all on the whole-level kernels runs the control in those kernels
     const bool fold_control = !d.n_sor && !d.n_units && (d.n_level || d.n_clus);
     for (int outer = 0; outer < P.hp.n_outer; outer++) {

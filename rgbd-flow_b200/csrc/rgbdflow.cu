@@ -252,6 +252,7 @@ std::string topo_key(const Plan<T, S>& P, const HostParams& hp, int tag, bool de
         k += std::to_string(P.steps[i].n_items > 0) + std::to_string(P.sor_cfg[i].K) + std::to_string(P.sor_cfg[i].nbuf) +
              std::to_string(P.sor_cfg[i].ilp) + (P.steps[i].n_sor > 0 ? "t" : "") + (P.steps[i].n_units > 0 ? "s" : "") +
              (P.steps[i].n_level > 0 ? "l" : "") + (P.steps[i].regs ? "w" : "") +
+             (P.steps[i].band_c ? "b" + std::to_string(P.steps[i].band_c) : "") +
              (P.steps[i].n_res > 0 ? "r" + std::to_string((P.steps[i].n_res + kResItems - 1) / kResItems) : "") +
              (P.steps[i].n_clus > 0 ? "c" + std::to_string(P.steps[i].clus_c) + "r" + std::to_string(P.steps[i].clus_kp) : "") + ".";
     const std::vector<PairSpec> none;
@@ -484,6 +485,7 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
         if (!P0.steps[sidx].regs) continue;
         SorChoice ch;
         ch.res_k = std::max(1, P0.steps[sidx].res_k);
+        ch.band_c = P0.steps[sidx].band_c;
         tt.m["r" + P0.step_keys[sidx]] = ch;
     }
     if (todo.empty()) {
@@ -1403,7 +1405,8 @@ int rgbdflow_autotune_describe(int device, char* buf, size_t len)
                 lay += " H" + std::to_string(e.first) + ":";
                 for (size_t q = 0; q < e.second.size(); q++) lay += (q ? "/" : "") + std::to_string(e.second[q]);
             }
-            if (ch.res_k) std::snprintf(b, sizeof b, "%s registers, exchange every %d; ", kv.first.c_str() + 1, ch.res_k);
+            if (ch.band_c) std::snprintf(b, sizeof b, "%s registers, bands of %d; ", kv.first.c_str() + 1, ch.band_c);
+            else if (ch.res_k) std::snprintf(b, sizeof b, "%s registers, exchange every %d; ", kv.first.c_str() + 1, ch.res_k);
             else if (ch.strip && !ch.bands.empty())
                 std::snprintf(b, sizeof b, "%s strip bands%s K %d %.2f us/it; ", kv.first.c_str(), lay.c_str(), ch.K, ch.us_per_it);
             else if (ch.strip) std::snprintf(b, sizeof b, "%s strip band %d K %d %.2f us/it; ", kv.first.c_str(), ch.seg, ch.K, ch.us_per_it);
