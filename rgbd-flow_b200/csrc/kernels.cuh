@@ -13,6 +13,8 @@
 #include <cooperative_groups.h>
 #include <stdint.h>
 
+#include "exact_math.cuh"
+
 namespace rgbdflow {
 
 constexpr int kMaxChecks = 512;  // SOR convergence checks per inner iteration (nSOR / period)
@@ -147,10 +149,6 @@ __device__ __forceinline__ float absT(float a) { return fabsf(a); }
 __device__ __forceinline__ double absT(double a) { return ::fabs(a); }
 __device__ __forceinline__ float expT(float a) { return expf(a); }
 __device__ __forceinline__ double expT(double a) { return ::exp(a); }
-
-template <class T> __device__ __forceinline__ T rsqrtT(T v);
-template <> __device__ __forceinline__ float rsqrtT<float>(float v) { return 1.0f / sqrtf(v); }
-template <> __device__ __forceinline__ double rsqrtT<double>(double v) { return 1.0 / sqrt(v); }
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
@@ -711,7 +709,9 @@ __device__ __forceinline__ void lin_phi_px(const LevelItem<T, S>& it, const Solv
     }
     const T s = __ldg(it.pyr[9] + gi * it.W + gj);
     const T q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3] + s * (d[4] * d[4] + d[5] * d[5]);
-    sv.at(kLinPhi, gi, gj) = (T)0.5 * rsqrtT<T>(q + k.eps_s);
+    T r[1] = {q + k.eps_s};
+    inv_sqrt<T, 1>(r, r);
+    sv.at(kLinPhi, gi, gj) = (T)0.5 * r[0];
 }
 
 // The system of pixel (gi, gj): o[0..11] (the sys planes), and of its left and upper edge the weight (sys[9] /
@@ -731,8 +731,8 @@ __device__ __forceinline__ void lin_system_px(const LevelItem<T, S>& it, const S
             sx += gfl[m] * sv.at(kLinB + c, gi, cc);
             sy += gfl[m] * sv.at(kLinB + c, rr, gj);
         }
-        Ix[c] = sx / (T)12;
-        Iy[c] = sy / (T)12;
+        Ix[c] = div_small<12>(sx);
+        Iy[c] = div_small<12>(sy);
         It[c] = sv.at(kLinDT + c, gi, gj);
     }
     Ix[5] = minT(maxT(Ix[5], -k.max_grad), k.max_grad);
@@ -742,20 +742,26 @@ __device__ __forceinline__ void lin_system_px(const LevelItem<T, S>& it, const S
     const T du0 = sv.at(kLinUD, gi, gj) - U0, du1 = sv.at(kLinUD + 1, gi, gj) - U1, du2 = sv.at(kLinUD + 2, gi, gj) - U2;
     const T z1 = ldS<T, S>(it.D1 + l);
     const T q = (z1 + U2 < ldS<T, S>(it.D2 + l) + k.occ_margin * (z1 * z1)) ? (T)1 : k.occ_penalty;
-    T sxy = 0, sx2 = 0, sy2 = 0, stx = 0, sty = 0;
+    T rs[6];
     for (int c = 0; c < 5; c++) {
         const T e = (It[c] + Ix[c] * du0 + Iy[c] * du1) * q;
-        const T psi = (T)0.5 * rsqrtT<T>(e * e + k.eps_d) * k.color_w;
+        rs[c] = e * e + k.eps_d;
+    }
+    const T e2 = It[5] + Ix[5] * du0 + Iy[5] * du1 - du2;
+    rs[5] = e2 * e2 + k.eps_z;
+    inv_sqrt<T, 6>(rs, rs);
+    T sxy = 0, sx2 = 0, sy2 = 0, stx = 0, sty = 0;
+    for (int c = 0; c < 5; c++) {
+        const T psi = (T)0.5 * rs[c] * k.color_w;
         sxy += psi * Ix[c] * Iy[c];
         sx2 += psi * Ix[c] * Ix[c];
         sy2 += psi * Iy[c] * Iy[c];
         stx += psi * Ix[c] * It[c];
         sty += psi * Iy[c] * It[c];
     }
-    const T ixy = sxy / (T)5, ix2 = sx2 / (T)5, iy2 = sy2 / (T)5;
-    const T itx = stx * q * q / (T)5, ity = sty * q * q / (T)5;
-    const T e2 = It[5] + Ix[5] * du0 + Iy[5] * du1 - du2;
-    const T pi = (T)0.5 * rsqrtT<T>(e2 * e2 + k.eps_z) * __ldg(it.pyr[8] + l);
+    const T ixy = div_small<5>(sxy), ix2 = div_small<5>(sx2), iy2 = div_small<5>(sy2);
+    const T itx = div_small<5>(stx * q * q), ity = div_small<5>(sty * q * q);
+    const T pi = (T)0.5 * rs[5] * __ldg(it.pyr[8] + l);
     const T dxy = pi * Ix[5] * Iy[5], dx2 = pi * Ix[5] * Ix[5], dy2 = pi * Iy[5] * Iy[5];
     const T dtx = pi * Ix[5] * It[5], dty = pi * Iy[5] * It[5];
     // weighted Laplacians of u (not u + du) and edge weights
@@ -789,9 +795,10 @@ __device__ __forceinline__ void lin_system_px(const LevelItem<T, S>& it, const S
     if (hasD) { const T e = phi * rvl; sumXY += e; sumZ += e * s; }
     const T al = k.alpha, ga = k.gamma, mg = __ldg(it.mag + l);
     // reciprocals of the diagonal: the SOR multiplies instead of dividing
-    o[0] = (T)1 / (-(ix2 + dx2 + al * sumXY) - ga);
-    o[1] = (T)1 / (-(iy2 + dy2 + al * sumXY) - ga);
-    o[2] = (T)1 / (-(pi + al * sumZ) - ga * mg);
+    o[0] = -(ix2 + dx2 + al * sumXY) - ga;
+    o[1] = -(iy2 + dy2 + al * sumXY) - ga;
+    o[2] = -(pi + al * sumZ) - ga * mg;
+    inverse<T, 3>(o);
     o[3] = -ixy - dxy;
     o[4] = pi * Ix[5];
     o[5] = pi * Iy[5];
