@@ -607,34 +607,41 @@ void run_batch(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPa
     char* pin_desc = pin_in + in_b;
     char* pin_out = pin_desc + align_up(P.desc_bytes, 256);
     char* pin_ctl = pin_out + out_b;
-    // host inputs: page-locked caller buffers are copied by DMA directly, others through staging
-    std::vector<std::pair<const void*, std::pair<size_t, size_t>>> direct;  // (src, (arena off, bytes))
+    std::memcpy(pin_desc, P.desc.data(), P.desc_bytes);
+    cudaStream_t st = dev ? user_stream : c->stream;
     if (!dev)
+        for (const auto& p : pairs)
+            for (const auto& seg : p.inputs())
+                if (!seg.first) throw ArgError(RGBDFLOW_ERR_INVALID_ARG, "pair " + std::to_string(&p - pairs.data()) + ": null input buffer");
+    if (c->pending) RF_CUDA(cudaStreamWaitEvent(st, c->done, 0));  // arena reuse across streams
+    if (!dev) {
+        // host inputs: page-locked caller buffers are copied by DMA directly, others through staging, the device's
+        // copy of what is staged (from half a megabyte) running while the rest is being staged
+        std::vector<std::pair<const void*, std::pair<size_t, size_t>>> direct;  // (src, (arena off, bytes))
+        size_t up = 0, staged = 0;  // [up, staged) of the staging waits for its copy
+        auto flush = [&] {
+            if (staged > up) RF_CUDA(cudaMemcpyAsync(c->arena + P.in_off + up, pin_in + up, staged - up, cudaMemcpyHostToDevice, st));
+        };
         for (int p = 0; p < P.n; p++) {
             const auto segs = pairs[p].inputs();
             for (size_t q = 0; q < segs.size(); q++) {
-                if (!segs[q].first) throw ArgError(RGBDFLOW_ERR_INVALID_ARG, "pair " + std::to_string(p) + ": null input buffer");
-                if (is_pinned(segs[q].first)) direct.push_back({segs[q].first, {P.in_seg[p][q], segs[q].second}});
-                else std::memcpy(pin_in + (P.in_seg[p][q] - P.in_off), segs[q].first, segs[q].second);
+                const size_t off = P.in_seg[p][q] - P.in_off, bytes = segs[q].second;
+                if (is_pinned(segs[q].first)) {
+                    direct.push_back({segs[q].first, {P.in_seg[p][q], bytes}});
+                    continue;
+                }
+                // apart from the last ones (a direct input lies between), or enough for a copy of its own
+                if (off < staged || off - staged >= 256 || staged - up >= (512u << 10)) {
+                    flush();
+                    up = off;
+                }
+                std::memcpy(pin_in + off, segs[q].first, bytes);
+                staged = off + bytes;
             }
         }
-    std::memcpy(pin_desc, P.desc.data(), P.desc_bytes);
-    cudaStream_t st = dev ? user_stream : c->stream;
-    if (c->pending) RF_CUDA(cudaStreamWaitEvent(st, c->done, 0));  // arena reuse across streams
-    if (!dev) {
-        if (direct.empty()) {
-            RF_CUDA(cudaMemcpyAsync(c->arena + P.in_off, pin_in, P.in_bytes, cudaMemcpyHostToDevice, st));
-        } else {
-            for (int p = 0; p < P.n; p++) {
-                const auto segs = pairs[p].inputs();
-                for (size_t q = 0; q < segs.size(); q++)
-                    if (!is_pinned(segs[q].first))
-                        RF_CUDA(cudaMemcpyAsync(c->arena + P.in_seg[p][q], pin_in + (P.in_seg[p][q] - P.in_off),
-                                                segs[q].second, cudaMemcpyHostToDevice, st));
-            }
-            for (const auto& d : direct)
-                RF_CUDA(cudaMemcpyAsync(c->arena + d.second.first, d.first, d.second.second, cudaMemcpyHostToDevice, st));
-        }
+        flush();
+        for (const auto& d : direct)
+            RF_CUDA(cudaMemcpyAsync(c->arena + d.second.first, d.first, d.second.second, cudaMemcpyHostToDevice, st));
     }
     RF_CUDA(cudaMemcpyAsync(c->arena + P.desc_off, pin_desc, P.desc_bytes, cudaMemcpyHostToDevice, st));
     RF_CUDA(cudaEventRecord(c->desc_up, st));
