@@ -922,7 +922,7 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
                 for (int c = 0; c < 4; c++) it.feat[c] = (float*)h.feat[c];
                 for (int c = 0; c < 2; c++) it.bp[c] = (float*)h.bp[c];
                 its.push_back(it);
-                rf.push_back(rf.back() + 7 * H);
+                rf.push_back(rf.back() + hpb_row_threads(H));
                 cf.push_back(cf.back() + 7 * (W + 1));
             }
             typename Plan<T, S>::HpbStep d;
@@ -1689,7 +1689,7 @@ static int enqueue_hpb(const Plan<T, S>& P, char* base, cudaStream_t st, Prof* p
         const HpbItem<T>* items = (const HpbItem<T>*)(db + h.items_off);
         const Tile* lt = (const Tile*)(db + d.lin_tiles_off);
         k_hpb_normals<T><<<d.n_lin, LTW * LTH, 0, st>>>(items, lt);
-        k_hpb_rowsum<T><<<(h.row_threads + 127) / 128, 128, 0, st>>>(items, (const int*)(db + h.row_first_off), h.n_items);
+        k_hpb_rowsum<T><<<(h.row_threads + 127) / 128, 32 * kHpbRowWarps, 0, st>>>(items, (const int*)(db + h.row_first_off), h.n_items);
         k_hpb_colsum<T><<<(h.col_threads + 127) / 128, 128, 0, st>>>(items, (const int*)(db + h.col_first_off), h.n_items);
         k_hpb_halfdisk<T><<<d.n_lin, LTW * LTH, 0, st>>>(items, lt);
         k_hpb_prob<T><<<d.n_lin, LTW * LTH, 0, st>>>(items, lt);
