@@ -272,13 +272,15 @@ typedef struct rgbdflow_kernel_stat {
 
 int rgbdflow_profile(rgbdflow_ctx* ctx, int enable);
 
-/* SOR autotuner (no reference counterpart; the reference has one SOR kernel configuration).  The
- * first time a pyramid level with given pair sizes is solved on a device, each SOR configuration
- * (tile or strip kernel, sweeps per launch, lane mapping, strip band height) is timed on that
- * level with CUDA events and the fastest is kept for the life of the process; every configuration
- * gives the same flow bit for bit.  RGBDFLOW_AUTOTUNE=0 in the environment turns it off.  Writes
- * the choices made on `device` ("sizes kernel K ... us per SOR iteration; ...") into buf (len bytes,
- * NUL-terminated; either may be 0) and returns the full length. */
+/* SOR configurations (no reference counterpart; the reference has one SOR kernel configuration).  FP32
+ * levels that fit the device's registers run from them, by rule.  For the others (FP64, levels of more than
+ * about 390,000 pixels, SOR settings given explicitly are not tuned), the first time a pyramid level with given
+ * pair sizes is solved on a device, each configuration (tile or strip kernel, sweeps per launch, lane
+ * mapping, strip band height) is timed on that level with CUDA events and the fastest is kept for the life of the
+ * process.  Every configuration gives the same flow bit for bit.  RGBDFLOW_AUTOTUNE=0 in the environment
+ * turns the timing off.  Writes the choices made on `device` ("sizes registers, bands of N; sizes registers,
+ * exchange every K; sizes kernel K ... us per SOR iteration; ...") into buf (len bytes, NUL-terminated; either may
+ * be 0) and returns the full length. */
 int rgbdflow_autotune_describe(int device, char* buf, size_t len);
 /* Fills up to max entries; returns the number of kernel classes with launches. */
 int rgbdflow_profile_read(rgbdflow_ctx* ctx, rgbdflow_kernel_stat* out, int max);

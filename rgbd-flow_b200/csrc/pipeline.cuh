@@ -238,8 +238,8 @@ static inline bool sor_from_registers(const HostParams& hp)
     return sizeof(T) == 4 && sor_tunable(hp) && hp.sor_level && hp.level_reg && tags < 2e9;
 }
 
-// Whether a level is small enough for one CTA with a position a thread (k_sor_level_reg), which beats the
-// resident kernel's four rows a warp there: 30 iterations of 40x30 41 us against 44, of 10x7 26 against 35.
+// Whether a level is small enough for one CTA with a position a thread (k_sor_level_reg; for steps that
+// k_level_bands does not take), which beats the resident kernel's four rows a warp there: 30 iterations of 40x30 41 us against 44, of 10x7 26 against 35.
 static inline bool whole_ok(int H, int hwp)
 {
     return H * hwp <= kLevelRegMax && level_reg_smem_bytes<float>(H, hwp) <= 64 * 1024;

@@ -10,13 +10,9 @@
 //   * vertical neighbours are the thread's own rows, except across warps (each warp publishes the
 //     unknowns of its first and last row in shared memory after every half-sweep).
 // Every register index is a compile-time constant, because a block starts on an even row and column and
-// so the colour of each of its pixels is fixed.  Rows a and a + 2 of a column have one colour and form a
-// pair of the packed FP32 instructions (two IEEE operations each): the right and left, upper and lower
-// neighbours of such a pair are pairs of the same kind in the thread's other column and rows, so packing
-// costs one register move per unknown.  An update is then 18 packed operations, 6 minima and maxima and
-// about 6 others, where the shared-memory kernels spend about 100 instructions.  Every pixel's operations
-// and their order are the tile kernel's (the negated weights negate exactly), so the results are the same
-// bit for bit.
+// so the colour of each of its pixels is fixed.  Every pixel's operations and their order are the tile kernel's
+// (the negated weights negate exactly), so the results are the same bit for bit.  (The packed FP32 instructions
+// were tried for pairs of rows: two operations in one take the register reads of two.)
 #pragma once
 #include "kernels.cuh"
 
@@ -201,7 +197,7 @@ __device__ __forceinline__ void reg_block_store(const RegBlock<V>& b, float* x, 
 // Measured, 30 iterations of one level (one pair): 640x480 91 us (tile SOR 261), 320x240 64 (108), 160x120 63
 // and 80x60 63 (cluster whole-level kernel 126 and 105); 16 pairs: 640x480 15.4 -> 9.1 ms of SOR a solve (strip
 // SOR), 320x240 3.3 -> 1.6 (strips), 160x120 0.81 -> 0.44 (cluster).  Levels of more than 148 tiles (about
-// 390,000 pixels) stay on the strip and tile SOR.
+// 390,000 pixels) stay on the strip and tile SOR, steps of few small levels go to k_level_bands.
 //
 // Items take the launch's CTAs in order, as many together as fit; a CTA goes through its items in order,
 // so an item waits for nothing but earlier items.
