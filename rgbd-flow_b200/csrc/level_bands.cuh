@@ -125,7 +125,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
     const int PLS = (B + 2) * 2 * RP;
     float* const xs = band_smem + kLinN * sv.n;  // the increment: [u, v, w][row + 1][colour][position + 1], zeros around
     float* const part = xs + 3 * PLS;            // the statistic of each tile's 16 warps, then of the tiles
-    const bool judge = it.allow_early && !k.fixed;
+    const bool stat = it.allow_early && !k.fixed;
     // this thread's position: local row li, half-row index m
     const int li = tid / hw, m = tid % hw, i = r0 + li;
     const bool inpos = tid < nr * hw;
@@ -158,7 +158,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
     float fz[2];
 #pragma unroll
     for (int c = 0; c < 2; c++)
-        fz[c] = judge && valid[c] ? divR(it.f_level, it.pyr[6][(size_t)i * W + 2 * m + (c ^ odd)]) : 0.f;
+        fz[c] = stat && valid[c] ? divR(it.f_level, it.pyr[6][(size_t)i * W + 2 * m + (c ^ odd)]) : 0.f;
     float cf[2][9], aL[2], aU[2], aR[2], aD[2], wL[2], wU[2], wR[2], wD[2], xp[2][3];
     bool ran = false;
     for (int outer = 0; outer < n_outer; outer++) {
@@ -298,7 +298,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
                     u[v] = addR(sv.at(kLinU + v, i, j), xp[c][v]);
                     sv.at(kLinU + v, i, j) = u[v];
                 }
-                if (judge)
+                if (stat)
                     sv.at(kLinPhi, i, j) = addR(addR(mulR(xp[c][0], xp[c][0]), mulR(xp[c][1], xp[c][1])),
                                                 mulR(mulR(xp[c][2], xp[c][2]), fz[c]));
                 if (to_up && li < 2)
@@ -311,7 +311,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
             }
         cluster_sync<CL>();
         float tot = 0.f;  // the statistic, on one lane
-        if (judge) {
+        if (stat) {
             // in the tile kernels' order: virtual thread vt (0..511) takes pixels vt and vt + 512 of the 32 x 32
             // tile, a warp tree per virtual warp, then the 16 virtual warps in order; every CTA gets every warp's
             for (int q = rank * n_warps + warp; q < tiles * 16; q += C * n_warps) {
