@@ -364,8 +364,10 @@ k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float>
 #pragma unroll 1
             for (int h = 0; h < 2 * nit; h++) {
                 if ((chk && h >= 2 * nit - 2) || L.masked) {
-                    if (h & 1) reg_half_sweep<kResV, 1, true>(b, up, down, own, k.omega, k.step, in, mine, md);
-                    else reg_half_sweep<kResV, 0, true>(b, up, down, own, k.omega, k.step, in, mine, md);
+                    // a check is of its own iteration, also where every one is masked
+                    const unsigned cnt = h >= 2 * nit - 2 ? mine : 0u;
+                    if (h & 1) reg_half_sweep<kResV, 1, true>(b, up, down, own, k.omega, k.step, in, cnt, md);
+                    else reg_half_sweep<kResV, 0, true>(b, up, down, own, k.omega, k.step, in, cnt, md);
                 } else {
                     if (h & 1) reg_half_sweep<kResV, 1, false>(b, up, down, own, k.omega, k.step, in, mine, md);
                     else reg_half_sweep<kResV, 0, false>(b, up, down, own, k.omega, k.step, in, mine, md);
