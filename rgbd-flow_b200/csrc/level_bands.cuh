@@ -29,6 +29,10 @@ namespace rgbdflow {
 constexpr int kBandMax = 640;    // positions of a band (threads of a CTA)
 constexpr int kBandSmall = 256;  // threads up to which a thread may keep 255 registers
 constexpr size_t kBandSmem = 200 * 1024;
+// Sets of the CTAs' largest changes that the convergence checks alternate between.  A check's barrier orders the
+// stores of the check after the next behind its reads, but not the next one's: until then only the neighbours' rows
+// tie the CTAs together, so that one d bands away may be d half-sweeps ahead of a warp that still reads.
+constexpr int kBandCheckSets = 2;
 
 // Row pitch (positions) of a half-row of the increment: a zero position each side, and the threads of a warp, which
 // span rows where hw < 32, on different banks.
@@ -108,7 +112,7 @@ __global__ void __launch_bounds__(NTM, 1)
 k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int n_outer, int n_inner, int* status)
 {
     extern __shared__ __align__(16) float band_smem[];
-    __shared__ float s_all[16], red[32];
+    __shared__ float s_all[kBandCheckSets][16], red[32];
     __shared__ __align__(8) unsigned long long s_mbar[2];  // the neighbours' rows of even and odd half-sweeps
     const int rank = CL ? (int)blockIdx.x % C : 0;
     // the item from shared memory: a cluster barrier drops what L1 holds of global memory
@@ -144,6 +148,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
         mbar_init(mbar + 8);
     }
     unsigned sweeps = 0;  // half-sweeps so far
+    int set = 0;          // of the next check's changes
     bool lost = false;    // a wait gave up
     auto await = [&](unsigned n) {
         if (!lost) lost = !mbar_wait(mbar + 8 * (n & 1), (n >> 1) & 1);
@@ -273,12 +278,13 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
                     if (tid < C) {
                         float g = 0.f;
                         for (int w = 0; w < n_warps; w++) g = fmaxf(g, red[w]);
-                        if (CL) cluster_store(cluster_addr(&s_all[rank], tid), g);
-                        else s_all[0] = g;
+                        if (CL) cluster_store(cluster_addr(&s_all[set][rank], tid), g);
+                        else s_all[set][0] = g;
                     }
                     cluster_sync<CL>();
                     float g = 0.f;
-                    for (int r = 0; r < C; r++) g = fmaxf(g, s_all[r]);
+                    for (int r = 0; r < C; r++) g = fmaxf(g, s_all[set][r]);
+                    set = (set + 1) % kBandCheckSets;
                     const bool stop = (double)g < k.sor_tol || g >= k.step;
                     if (g > 0) maxdiff = g;
                     if (stop) iters = itn + 1;
