@@ -83,10 +83,11 @@ __device__ __forceinline__ void mbar_expect(unsigned mbar, int bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
-// Waits (bounded: about a second) for the phase of the given parity; false: it gave up.
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, int parity)
+// Waits (`polls` tries) for the phase of the given parity; false: it gave up.
+constexpr int kBandPolls = 1 << 20;
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, int parity, int polls)
 {
-    for (int p = 0; p < (1 << 20); p++) {
+    for (int p = 0; p < polls; p++) {
         int ok;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
                      " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
@@ -106,10 +107,19 @@ __device__ __forceinline__ void cluster_sync()
     }
 }
 
+// The end of a block (all its threads) of which some may have lost a wait: reports it, and stays for a millisecond so
+// that rows the neighbours sent before the last cluster barrier land in shared memory that is still this block's.
+__device__ __forceinline__ void report_lost(bool lost, int* status)
+{
+    if (!__syncthreads_or(lost)) return;
+    report_wait_failure(status);
+    for (int q = 0; q < 16; q++) __nanosleep(65536);
+}
+
 // NTM: most threads of a CTA.  CL: more than one CTA an item.
 template <class S, int NTM, bool CL>
 __global__ void __launch_bounds__(NTM, 1)
-k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int n_outer, int n_inner, int* status)
+k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int n_outer, int n_inner, int polls, int* status)
 {
     extern __shared__ __align__(16) float band_smem[];
     __shared__ float s_all[kBandCheckSets][16], red[32];
@@ -149,9 +159,16 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
     }
     unsigned sweeps = 0;  // half-sweeps so far
     int set = 0;          // of the next check's changes
-    bool lost = false;    // a wait gave up
+    // the thread's row goes to the band above / below; it arrives at the block's barriers (a thread that also waits)
+    bool send_up = to_up && li == 0, send_dn = to_dn && li == nr - 1, expects = CL && tid == (to_up ? 0 : (nr - 1) * hw);
+    // A wait gave up: from then on the thread neither waits nor sends nor arrives (the barrier's last phase may be
+    // open), and only the cluster barriers go on.
+    bool lost = false;
     auto await = [&](unsigned n) {
-        if (!lost) lost = !mbar_wait(mbar + 8 * (n & 1), (n >> 1) & 1);
+        if (!lost && !mbar_wait(mbar + 8 * (n & 1), (n >> 1) & 1, polls)) {
+            lost = true;
+            send_up = send_dn = expects = false;
+        }
     };
 
     for (int q = tid; q < (nr + 4) * W; q += NT) {
@@ -231,8 +248,8 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
                 for (int c = 0; c < 2; c++) {
                     if (CL) {
                         // the row of a neighbour that the half-sweep before has sent
-                        if (itn + c > 0 && ((to_up && li == 0) || (to_dn && li == nr - 1))) await(sweeps - 1);
-                        if (tid == 0)
+                        if (itn + c > 0 && (send_up || send_dn)) await(sweeps - 1);
+                        if (expects)
                             mbar_expect(mbar + 8 * (sweeps & 1), 12 * ((to_up ? (W + 1 - (c ^ ((r0 + 1) & 1))) / 2 : 0) +
                                                                       (to_dn ? (W + 1 - (c ^ ((r0 + nr) & 1))) / 2 : 0)));
                     }
@@ -256,12 +273,12 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
                             if (chk) md = fmaxf(md, fabsf(nv[v] - xp[c][v]));
                             xp[c][v] = nv[v];
                         }
-                        if (to_up && li == 0) {
+                        if (send_up) {
                             const int o = xs0 + ((nr_up + 1) * 2 + c) * RP + m + 1;
 #pragma unroll
                             for (int v = 0; v < 3; v++) cluster_send(base_up + 4 * (o + v * PLS), nv[v], mbar_up + 8 * (sweeps & 1));
                         }
-                        if (to_dn && li == nr - 1) {
+                        if (send_dn) {
                             const int o = xs0 + c * RP + m + 1;
 #pragma unroll
                             for (int v = 0; v < 3; v++) cluster_send(base_dn + 4 * (o + v * PLS), nv[v], mbar_dn + 8 * (sweeps & 1));
@@ -355,7 +372,7 @@ k_level_bands(const LevelItem<float, S>* items, SolveConst<float> k, int C, int 
         if (rank == 0 && tid == 0) control_record(it, k, outer, tot, iters, maxdiff, done);
         if (done) break;
     }
-    if (lost && status) report_wait_failure(status);
+    if (CL) report_lost(lost, status);
     if (!ran) return;
     // ---- the flow, and the last system for rgbdflow_debug_read_plane
 #pragma unroll

@@ -147,6 +147,7 @@ struct HostParams {
     int level_cluster;                        // > 1: such levels run on a cluster of this many CTAs instead
     int level_reg;                            // FP32 whole-level SOR with the system in registers (0: off)
     int res_k;                                // iterations between the resident SOR's exchanges (0: resident_k())
+    int wait_polls;                           // polls after which the SOR's waits give up (-1: each kernel's own limit)
 };
 
 // Row pitch of the u planes, and the checkerboard half-row length of the x / sys planes (16-byte
@@ -1550,7 +1551,8 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
             const bool small = d.band_threads <= kBandSmall;
             auto* const kernel = d.band_c > 1 ? (small ? k_level_bands<S, kBandSmall, true> : k_level_bands<S, kBandMax, true>)
                                               : (small ? k_level_bands<S, kBandSmall, false> : k_level_bands<S, kBandMax, false>);
-            RF_CUDA(cudaLaunchKernelEx(&cfg, kernel, items, k, d.band_c, P.hp.n_outer, P.hp.n_inner, P.status));
+            RF_CUDA(cudaLaunchKernelEx(&cfg, kernel, items, k, d.band_c, P.hp.n_outer, P.hp.n_inner,
+                                       P.hp.wait_polls >= 0 ? P.hp.wait_polls : kBandPolls, P.status));
             RF_PROF_E(pf, st);
             return launches + 1;
         }

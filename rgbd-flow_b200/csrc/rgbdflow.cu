@@ -192,6 +192,8 @@ HostParams host_params(const rgbdflow_params& p)
     h.level_reg = e ? std::atoi(e) : 1;
     e = std::getenv("RGBDFLOW_RESIDENT_K");
     h.res_k = e ? std::atoi(e) : 0;
+    e = std::getenv("RGBDFLOW_WAIT_POLLS");
+    h.wait_polls = e ? std::max(0, std::atoi(e)) : -1;
     h.fill_rounds = 253;  // round stamps are bytes: 0 valid, 1..253 rounds, 254 outside, 255 unfilled
     return h;
 }
@@ -235,8 +237,8 @@ std::string plan_key(const std::vector<PairSpec>& ps, const HostParams& hp, int 
                   hp.n_sor, hp.max_dist, hp.fill_holes, hp.fixed, hp.omega, hp.step, hp.eps_d, hp.eps_z, hp.eps_s,
                   hp.sor_tol, hp.outer_tol, hp.occ_margin, hp.occ_penalty, hp.max_grad, hp.period, hp.K * 100 + hp.sor_ilp * 10 + hp.sor_nbuf, hp.fill_rounds);
     k += buf;
-    std::snprintf(buf, sizeof buf, " strip %d %d %d %d %ld %d level %d %d %d r %d", hp.sor_strip, hp.strip_min_w, hp.strip_min_h,
-                  hp.strip_seg, hp.strip_min_px, hp.strip_balanced, hp.sor_level, hp.level_cluster, hp.level_reg, hp.res_k);
+    std::snprintf(buf, sizeof buf, " strip %d %d %d %d %ld %d level %d %d %d r %d p %d", hp.sor_strip, hp.strip_min_w, hp.strip_min_h,
+                  hp.strip_seg, hp.strip_min_px, hp.strip_balanced, hp.sor_level, hp.level_cluster, hp.level_reg, hp.res_k, hp.wait_polls);
     return k + buf;
 }
 

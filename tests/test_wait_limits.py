@@ -1,0 +1,49 @@
+"""Waits between thread blocks that run out: the call that waited reports it, and the context stays usable.
+
+RGBDFLOW_WAIT_POLLS=0 makes every such wait of the SOR give up at once.  Nothing hangs and no access leaves its
+buffers: the blocks go on with what they have, or return.
+"""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import rgbdflow as rf
+from test_resident_tiles import pair
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+TIMEOUT = -5  # RGBDFLOW_ERR_TIMEOUT
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc to compile the probe")
+def test_a_wait_lost_by_any_thread_is_reported(tmp_path):
+    exe = str(tmp_path / "lost_wait_check")
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                    os.path.join(HERE, "cpp", "lost_wait_check.cu")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def solve(ctx, W=160, H=120):
+    p = pair(W, H, 3)
+    cam = rf.CameraParams.make(W, H, p["cam"].f, p["cam"].cx, p["cam"].cy)
+    return ctx.scene_flow_two_frames(cam, p["bgr1"], p["depth1"], p["bgr2"], p["depth2"], rf.benchmark_params(W), stats=False)
+
+
+def assert_reported_once(ctx, monkeypatch):
+    before = solve(ctx)
+    monkeypatch.setenv("RGBDFLOW_WAIT_POLLS", "0")
+    with pytest.raises(rf.RgbdFlowError) as e:
+        solve(ctx)
+    assert e.value.code == TIMEOUT
+    monkeypatch.delenv("RGBDFLOW_WAIT_POLLS")
+    ctx.synchronize()
+    np.testing.assert_array_equal(solve(ctx), before)
+
+
+@pytest.mark.gpu
+def test_level_bands_report_lost_waits(ctx, monkeypatch):
+    assert_reported_once(ctx, monkeypatch)
