@@ -1500,8 +1500,10 @@ static int enqueue_sor_regs(const Plan<T, S>& P, char* base, int sidx, cudaStrea
     const ResItem* ri = (const ResItem*)(base + P.desc_off + d.res_items_off);
     RF_PROF_B(pf, KC_SOR_LEVEL0 + lvl, st);
     for (int i = 0; i < d.n_res; i += kResItems) {
-        launch_cooperative(k_sor_resident, std::min(P.sms, d.res_tiles), kResNT, st, ri + i, std::min(kResItems, d.n_res - i), k, L,
-                           (unsigned)(outer * P.hp.n_inner + hh) * (unsigned)(P.hp.n_sor + 1), P.status);
+        const int n = std::min(kResItems, d.n_res - i);
+        launch_cooperative(k_sor_resident, std::min(P.sms, d.res_tiles), kResNT, st, ri + i, n, k, L,
+                           (unsigned)(outer * P.hp.n_inner + hh) * (unsigned)(P.hp.n_sor + 1),
+                           P.hp.wait_polls >= 0 ? P.hp.wait_polls : resident_polls(n, P.hp.n_sor), P.status);
         launches++;
     }
     if (last) {

@@ -274,13 +274,20 @@ __device__ __forceinline__ void load_word(const ulonglong2* p, bool want, unsign
                  " @w ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
                  : "=l"(lo), "=l"(hi) : "l"(p), "r"((unsigned)want), "l"(0ull) : "memory");
 }
-// Polls of a word or counter before a wait gives up (about a second).
-constexpr int kResPolls = 1 << 20;
+// Polls of a word or counter before a wait gives up (0.35 us or more each, so a third of a second at least), and what
+// a launch adds for each SOR iteration of each item but one: a tile's neighbours may still be at earlier items, and
+// an iteration takes them up to 5 us.
+constexpr int kResPolls = 1 << 20, kResPollsIteration = 16;
+static inline int resident_polls(int n_items, int n_sor)
+{
+    const double p = kResPolls + (double)kResPollsIteration * (n_items - 1) * n_sor;
+    return p < (1 << 30) ? (int)p : 1 << 30;
+}
 
 // tag0: the launch's first tag less one; a launch uses at most n_sor of them.
 __global__ void __launch_bounds__(kResNT, 1)
 k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float> k, SorLaunch L, unsigned tag0,
-               int* status)
+               int polls, int* status)
 {
     __shared__ float ex[(kResW + 2) * kRegEx];  // slot w + 1: warp w; slots 0 and 13 stay 0
     __shared__ int s_first[kResItems], s_tiles[kResItems];  // the CTAs of each item: first and number (0: done)
@@ -400,8 +407,8 @@ k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float>
                     atomicAdd(&ctl->arrived, 1u);
                     const unsigned want = (unsigned)t.tiles * (unsigned)(itn / k.period);
                     int p = 0;
-                    while (*(volatile unsigned*)&ctl->arrived < want && ++p < kResPolls) {}
-                    ok = p < kResPolls;
+                    while (*(volatile unsigned*)&ctl->arrived < want && ++p < polls) {}
+                    ok = p < polls;
                     __threadfence();
                     s_max = __ldcg(&ctl->maxdiff[ci]);
                 }
@@ -423,7 +430,7 @@ k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float>
             }
             // all of a thread's words in flight together (two at a time took 2.1 us instead of 0.9)
             unsigned halo = in & ~mine;
-            for (int p = 0; __any_sync(0xffffffffu, halo != 0) && p < kResPolls; p++) {
+            for (int p = 0; __any_sync(0xffffffffu, halo != 0) && p < polls; p++) {
                 unsigned long long lo[2 * kResV], hi[2 * kResV];
 #pragma unroll
                 for (int q = 0; q < 2 * kResV; q++)

@@ -27,6 +27,15 @@ def test_a_wait_lost_by_any_thread_is_reported(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc to compile the pipeline header")
+def test_resident_waits_outlast_the_items_queued_before(tmp_path):
+    exe = str(tmp_path / "resident_waits_check")
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                    os.path.join(HERE, "cpp", "resident_waits_check.cu")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def solve(ctx, W=160, H=120):
     p = pair(W, H, 3)
     cam = rf.CameraParams.make(W, H, p["cam"].f, p["cam"].cx, p["cam"].cy)
@@ -46,4 +55,11 @@ def assert_reported_once(ctx, monkeypatch):
 
 @pytest.mark.gpu
 def test_level_bands_report_lost_waits(ctx, monkeypatch):
+    assert_reported_once(ctx, monkeypatch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1, 5])
+def test_resident_sor_reports_lost_waits(ctx, monkeypatch, K):
+    monkeypatch.setenv("RGBDFLOW_RESIDENT_K", str(K))
     assert_reported_once(ctx, monkeypatch)
