@@ -750,6 +750,7 @@ static bool prepare_batch(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, c
     Plan<T, S> P = plan_for<T, S>(c, pairs, hp);
     if (c->graphs.count(graph_key(pairs, hp, slot, true, P.tune_desc))) return true;
     P.sms = c->sms;
+    P.status = c->dev_status;
     if (!c->arena || P.arena_bytes > c->arena_cap) return false;
     bind_plan(P, c->arena);
     graph_for(c, P, pairs, hp, slot, true);

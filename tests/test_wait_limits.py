@@ -63,3 +63,22 @@ def test_level_bands_report_lost_waits(ctx, monkeypatch):
 def test_resident_sor_reports_lost_waits(ctx, monkeypatch, K):
     monkeypatch.setenv("RGBDFLOW_RESIDENT_K", str(K))
     assert_reported_once(ctx, monkeypatch)
+
+
+@pytest.mark.gpu
+def test_served_batches_report_lost_waits(ctx, monkeypatch):
+    """A server captures its streams' batches ahead of their first launch: those carry the status too."""
+    monkeypatch.setenv("RGBDFLOW_WAIT_POLLS", "0")
+    W, H = 160, 120
+    frames = [pair(W, H, 90 + k) for k in range(4)]
+    cam = rf.CameraParams.make(W, H, frames[0]["cam"].f, frames[0]["cam"].cx, frames[0]["cam"].cy)
+    srv = rf.Server(ctx, rf.benchmark_params(W), max_streams=2, max_batch=2, warm_start=False)
+    status = []
+    try:
+        for k, f in enumerate(frames):
+            srv.submit(0, k, cam, f["bgr1"], f["depth1"])
+            while srv.pending():
+                status += [r[5] for r in srv.step(wait=True)]
+    finally:
+        srv.close()
+    assert status == [TIMEOUT] * 3
