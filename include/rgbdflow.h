@@ -249,7 +249,7 @@ int rgbdflow_scene_flow_batch_submit(rgbdflow_ctx* ctx, const rgbdflow_pair* pai
                                      const rgbdflow_params* params);
 
 /* Wait for every solve this context enqueued (on any stream).  The device's bounded waits (the
- * grid barriers of the cooperative hole-fill kernels) record a wait that gave up in a status word
+ * grid barriers of the hole-fill kernels, the SOR's between thread blocks) record a wait that gave up in a status word
  * of the context: synchronous calls return RGBDFLOW_ERR_TIMEOUT for it, and for submitted or
  * device-pointer solves this call does (once; the word is then cleared). */
 int rgbdflow_ctx_synchronize(rgbdflow_ctx* ctx);
@@ -409,6 +409,8 @@ int rgbdflow_server_counters_read(rgbdflow_server* srv, int reset, rgbdflow_serv
  *   Overlap: all calls on a device share the one workspace.  Two calls whose work overlaps on
  *   the device (different streams, or threads without ordering) race and corrupt each other's
  *   results; keep them on one stream, or order them with events.
+ *   Lost waits: the call returns before the solve has run and has no context, so a bounded device
+ *   wait that gives up (RGBDFLOW_ERR_TIMEOUT elsewhere) makes every component of flow_out NaN.
  *   err / err_len: NULL or a buffer that receives the error message.
  * ------------------------------------------------------------------------------------------- */
 int rgbdflow_scene_flow_noalloc(const rgbdflow_pair* pair, const rgbdflow_params* params, void* stream,

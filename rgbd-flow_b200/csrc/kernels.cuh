@@ -2322,9 +2322,10 @@ __global__ void k_control(const LevelItem<T, S>* items, int n_items, SolveConst<
     control_item(items[w], k, outer, n_checks, threadIdx.x & 31);
 }
 
-// Final flow (level 0) to the caller's interleaved (u, v, w) float layout.
+// Final flow (level 0) to the caller's interleaved (u, v, w) float layout.  lost: null, or a word that is set where a
+// wait of the solve gave up; the flow is NaN then.
 template <class T, class S>
-__global__ void k_output(const LevelItem<T, S>* items, const Tile* tiles, T* const* outs)
+__global__ void k_output(const LevelItem<T, S>* items, const Tile* tiles, T* const* outs, const int* lost)
 {
     const Tile t = tiles[blockIdx.x];
     const LevelItem<T, S>& it = items[t.item];
@@ -2333,9 +2334,8 @@ __global__ void k_output(const LevelItem<T, S>* items, const Tile* tiles, T* con
     const int l = i * it.W + j;
     T* o = outs[t.item];
     const int lp = i * it.pitch + j;
-    o[(size_t)l * 3 + 0] = it.u[0][lp];
-    o[(size_t)l * 3 + 1] = it.u[1][lp];
-    o[(size_t)l * 3 + 2] = it.u[2][lp];
+    const bool bad = lost && *lost;
+    for (int c = 0; c < 3; c++) o[(size_t)l * 3 + c] = bad ? (T)nanf("") : it.u[c][lp];
 }
 
 // Device warp of the final flow (for the single-scale seam's warpIm2 / warpDm2 outputs).

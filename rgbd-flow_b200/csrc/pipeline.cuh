@@ -542,7 +542,8 @@ struct Plan {
     size_t in_off = 0, in_bytes = 0;    // inputs uploaded each call (bgr, depth, est)
     size_t out_off = 0, out_bytes = 0;  // flows read back
     size_t ctl_off = 0;                 // PairCtl[n]
-    size_t ctr_off = 0;                 // int[16]: strip SOR ticket counter per step (zeroed with ctl)
+    size_t ctr_off = 0;                 // int[16]: strip SOR ticket counter per step, then the solve's own status word
+                                        // (zeroed with ctl)
     size_t desc_off = 0, desc_bytes = 0;
     int kind = 0;
     std::vector<std::vector<size_t>> in_seg;  // per pair: arena offset of each input segment
@@ -591,6 +592,7 @@ struct Plan {
     // HPB regularisation weights (regularization == HPB, kinds 0 and 1)
     bool hpb = false;
     int* status = nullptr;              // the context's device status word (bounded waits that gave up)
+    bool status_in_flow = false;        // no context: a wait that gave up turns the flow to NaN
     size_t hpb_ctr_off = 0;             // int[2n] region / pixel counts, then the fill's GridSync (zeroed each solve)
     size_t hpb_fill_off = 0;            // HpbFill[n] (descriptor offset)
     struct HpbDepthLevel { size_t jobs_off; int n_jobs; size_t tiles_off; int n_tiles; };
@@ -672,8 +674,8 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         }
     Bump A;
     P.ctl_off = A.take(sizeof(PairCtl) * P.n);
-    P.ctr_off = A.take(sizeof(int) * (16 + 256) + sizeof(GridSync));
-    P.unfilled_off = P.ctr_off + sizeof(int) * 16;
+    P.ctr_off = A.take(sizeof(int) * (17 + 256) + sizeof(GridSync));
+    P.unfilled_off = P.ctr_off + sizeof(int) * 17;
     {
         size_t nt = 0;
         for (const auto& p : pairs) nt += (size_t)((p.W + LTW - 1) / LTW) * ((p.H + LTH - 1) / LTH);
@@ -1711,7 +1713,7 @@ static int enqueue_solve(const Plan<T, S>& P, char* base, cudaStream_t st, Prof*
 {
     int launches = 0;
     char* db = base + P.desc_off;
-    RF_CUDA(cudaMemsetAsync(base + P.ctl_off, 0, P.ctr_off + sizeof(int) * 16 - P.ctl_off, st));  // ctl + tickets
+    RF_CUDA(cudaMemsetAsync(base + P.ctl_off, 0, P.ctr_off + sizeof(int) * 17 - P.ctl_off, st));  // ctl, tickets, status
     const auto& fin = P.steps.back();
     const LevelItem<T, S>* fin_items = (const LevelItem<T, S>*)(db + fin.items_off);
     const Tile* fin_tiles = (const Tile*)(db + fin.lin_tiles_off);
@@ -1773,7 +1775,8 @@ static int enqueue_solve(const Plan<T, S>& P, char* base, cudaStream_t st, Prof*
         for (int s = 0; s < P.Lmax; s++) launches += enqueue_level(P, base, s, st, 1, pf);
     }
     RF_PROF_B(pf, KC_OUT, st);
-    k_output<T, S><<<fin.n_lin, LTW * LTH, 0, st>>>(fin_items, fin_tiles, (T* const*)(db + P.out_ptrs_off));
+    k_output<T, S><<<fin.n_lin, LTW * LTH, 0, st>>>(fin_items, fin_tiles, (T* const*)(db + P.out_ptrs_off),
+                                                      P.status_in_flow ? P.status : nullptr);
     RF_PROF_E(pf, st);
     launches++;
     RF_CUDA(cudaGetLastError());

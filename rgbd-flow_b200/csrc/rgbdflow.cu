@@ -2057,6 +2057,9 @@ extern "C" int rgbdflow_scene_flow_noalloc(const rgbdflow_pair* pair, const rgbd
         if (dev < 0 || dev >= kNoAllocMaxDevices) throw ArgError(RGBDFLOW_ERR_UNSUPPORTED, "device index above 63");
         const NoAllocDevice& d = noalloc_setup(dev);
         P.sms = d.sms;
+        // no context's status word: the call's own, and what it says is in the flow
+        P.status = (int*)(d.scratch + P.ctr_off) + 16;
+        P.status_in_flow = true;
         bind_plan(P, d.scratch);
         unsigned char* db = P.desc.data();
         PrepItem<float>* prep = (PrepItem<float>*)(db + P.prep_items_off);

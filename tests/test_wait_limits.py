@@ -82,3 +82,28 @@ def test_served_batches_report_lost_waits(ctx, monkeypatch):
     finally:
         srv.close()
     assert status == [TIMEOUT] * 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", ["0", "2"])
+def test_a_lost_wait_of_the_allocation_free_solve_is_in_its_flow(monkeypatch, K):
+    import torch
+    W, H = 160, 120
+    p = pair(W, H, 3)
+    dev = {k: torch.from_numpy(np.ascontiguousarray(p[k])).cuda() for k in ("bgr1", "depth1", "bgr2", "depth2")}
+    q = dict(dev, W=W, H=H, cam=rf.CameraParams.make(W, H, p["cam"].f, p["cam"].cx, p["cam"].cy),
+             out=torch.zeros((H, W, 3), dtype=torch.float32, device="cuda"))
+    st = torch.cuda.Stream()
+
+    def flow():
+        rf.scene_flow_noalloc(q, rf.benchmark_params(W), stream=st)
+        st.synchronize()
+        return q["out"].cpu().numpy()
+
+    monkeypatch.setenv("RGBDFLOW_RESIDENT_K", K)  # 0: level bands and the rule's exchanges
+    before = flow()
+    assert np.isfinite(before).all()
+    monkeypatch.setenv("RGBDFLOW_WAIT_POLLS", "0")
+    assert np.isnan(flow()).all()
+    monkeypatch.delenv("RGBDFLOW_WAIT_POLLS")
+    np.testing.assert_array_equal(flow(), before)
