@@ -532,7 +532,7 @@ template <class T, class S>
 struct Plan {
     // ---- shape
     int n = 0, Lmax = 0;
-    int sms = 148;                // multiprocessors of the device (persistent SOR grid)
+    int sms = 0;                  // multiprocessors of the device
     std::vector<SorConfig> sor_cfg;  // SOR kernel configuration per step
     std::vector<PyrShape> shapes;
     std::vector<int> L;           // levels per pair
@@ -649,12 +649,16 @@ static inline std::vector<SorLaunch> sor_schedule(int nSOR, int K, int period, i
     return v;
 }
 
+// sms: the device's multiprocessors, which decide what a step's SOR can keep resident.
+constexpr int kPlanSms = 148;  // a B200's, for sizes asked without a device
 template <class T, class S>
-static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams& hp, const TuneTable* tune = nullptr)
+static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams& hp, const TuneTable* tune = nullptr,
+                            int sms = kPlanSms)
 {
     if (!sor_tunable(hp)) tune = nullptr;
     Plan<T, S> P;
     P.hp = hp;
+    P.sms = sms;
     P.n = (int)pairs.size();
     P.kind = pairs.empty() ? 0 : pairs[0].kind;
     for (const auto& p : pairs) {
@@ -992,7 +996,7 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         const SorChoice* ch = nullptr;
         // the step runs from registers when every item's level fits the device's
         std::vector<size_t> scratch;
-        const int ctas = P.sms > 0 ? P.sms : 148;
+        const int ctas = P.sms;
         bool regs = sor_from_registers<T>(hp);
         for (size_t q = 0, p = 0; q < items.size(); q++, p++) {
             while (k >= P.L[p]) p++;  // the item's pair
@@ -1057,7 +1061,7 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         if (ch) hs.strip_seg = ch->seg;
         BandMap bal;
         if (!ch && hp.strip_balanced && !strip_items.empty())
-            bal = strip_balanced_bands(items, strip_items, hp.strip_seg > 0 ? hp.strip_seg : 128, P.sms > 0 ? P.sms : 148);
+            bal = strip_balanced_bands(items, strip_items, hp.strip_seg > 0 ? hp.strip_seg : 128, P.sms);
         const std::vector<StripUnit> units = strip_units(items, strip_items, hs, P.sms, ch ? &ch->bands : &bal);
         if (ch) {
             P.tune_desc += skey + (ch->strip ? "s" + std::to_string(ch->seg) : "t") + std::to_string(ch->K) +

@@ -460,7 +460,7 @@ std::vector<SorChoice> sor_candidates(const Plan<T, S>& P, int sidx)
         }
         SorChoice ch;
         ch.strip = 1; ch.K = kStripMaxNit; ch.ilp = 2; ch.seg = 128;
-        ch.bands = strip_balanced_bands(items, which, 128, P.sms > 0 ? P.sms : 148);
+        ch.bands = strip_balanced_bands(items, which, 128, P.sms);
         bool differs = false;
         for (const auto& e : ch.bands) differs = differs || e.second != strip_default_bands(e.first, 128);
         if (differs) v.push_back(ch);
@@ -478,7 +478,7 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
     TuneTable& tt = ts.table[c->device & 63];
     const std::string bkey = plan_key(pairs, hp, (int)sizeof(T) * 10 + (int)sizeof(S));
     if (ts.complete[c->device & 63].count(bkey)) return;
-    const Plan<T, S> P0 = make_plan<T, S>(pairs, hp, &tt);
+    const Plan<T, S> P0 = make_plan<T, S>(pairs, hp, &tt, c->sms);
     std::vector<int> todo;
     for (int sidx = 0; sidx < P0.Lmax; sidx++)
         if (!P0.step_tuned[sidx] && (P0.steps[sidx].n_sor || P0.steps[sidx].n_units)) todo.push_back(sidx);
@@ -506,8 +506,7 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
         for (SorChoice cand : sor_candidates(P0, sidx)) {
             TuneTable one = tt;
             one.m[P0.step_keys[sidx]] = cand;
-            Plan<T, S> Pc = make_plan<T, S>(pairs, hp, &one);
-            Pc.sms = c->sms;
+            Plan<T, S> Pc = make_plan<T, S>(pairs, hp, &one, c->sms);
             ensure_arena(c, Pc.arena_bytes);
             bind_plan(Pc, c->arena);
             RF_CUDA(cudaMemcpy(c->arena + Pc.desc_off, Pc.desc.data(), Pc.desc_bytes, cudaMemcpyHostToDevice));
@@ -566,7 +565,7 @@ Plan<T, S> plan_for(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const H
     tune_sor<T, S>(c, pairs, hp);
     TuneState& ts = tune_state();
     std::lock_guard<std::mutex> lk(ts.mu);
-    return make_plan<T, S>(pairs, hp, autotune_enabled() ? &ts.table[c->device & 63] : nullptr);
+    return make_plan<T, S>(pairs, hp, autotune_enabled() ? &ts.table[c->device & 63] : nullptr, c->sms);
 }
 
 // Runs a batch through one graph launch.
@@ -580,7 +579,6 @@ void run_batch(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPa
     ensure_attrs<T, S>(c, slot);
     const bool dev = user_stream != nullptr;
     Plan<T, S> P = plan_for<T, S>(c, pairs, hp);
-    P.sms = c->sms;
     P.status = c->dev_status;
     ensure_arena(c, P.arena_bytes);
     bind_plan(P, c->arena);
@@ -749,7 +747,6 @@ static bool prepare_batch(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, c
     ensure_attrs<T, S>(c, slot);
     Plan<T, S> P = plan_for<T, S>(c, pairs, hp);
     if (c->graphs.count(graph_key(pairs, hp, slot, true, P.tune_desc))) return true;
-    P.sms = c->sms;
     P.status = c->dev_status;
     if (!c->arena || P.arena_bytes > c->arena_cap) return false;
     bind_plan(P, c->arena);
@@ -1705,25 +1702,25 @@ void server_retire(rgbdflow_server* s, ServerSlot& sl)
 struct SlotNeed {
     size_t arena = 0, pin = 0;
 };
-SlotNeed slot_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage)
+SlotNeed slot_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, int sms)
 {
     // the storage type changes plane sizes only, not the descriptor count
     size_t arena = 0, desc = 0;
     if (storage == RGBDFLOW_STORE_FP16) {
-        const auto P = make_plan<float, __half>(ps, hp);
+        const auto P = make_plan<float, __half>(ps, hp, nullptr, sms);
         arena = P.arena_bytes; desc = P.desc_bytes;
     } else if (storage == RGBDFLOW_STORE_BF16) {
-        const auto P = make_plan<float, __nv_bfloat16>(ps, hp);
+        const auto P = make_plan<float, __nv_bfloat16>(ps, hp, nullptr, sms);
         arena = P.arena_bytes; desc = P.desc_bytes;
     } else {
-        const auto P = make_plan<float, float>(ps, hp);
+        const auto P = make_plan<float, float>(ps, hp, nullptr, sms);
         arena = P.arena_bytes; desc = P.desc_bytes;
     }
     return SlotNeed{arena, align_up(desc, 256) + sizeof(PairCtl) * ps.size()};
 }
-size_t slot_arena_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage)
+size_t slot_arena_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, int sms)
 {
-    return slot_need(ps, hp, storage).arena;
+    return slot_need(ps, hp, storage, sms).arena;
 }
 
 // Arena bytes of a batch for admission: the sum of its pairs' single-pair arenas (an upper bound:
@@ -1734,9 +1731,9 @@ size_t admit_need(rgbdflow_server* s, const std::vector<PairSpec>& ps, const Hos
     size_t tot = 0;
     for (const auto& q : ps) {
         const std::string key = std::to_string(q.W) + "x" + std::to_string(q.H) + (q.warm() ? "w" : "c") +
-                                std::to_string(s->cfg.params.storage) + plan_key({}, hp, 0);
+                                std::to_string(s->cfg.params.storage) + "m" + std::to_string(s->ctx->sms) + plan_key({}, hp, 0);
         auto it = cache.find(key);
-        if (it == cache.end()) it = cache.emplace(key, slot_arena_need({q}, hp, s->cfg.params.storage)).first;
+        if (it == cache.end()) it = cache.emplace(key, slot_arena_need({q}, hp, s->cfg.params.storage, s->ctx->sms)).first;
         tot += it->second;
     }
     return tot;
@@ -1757,7 +1754,7 @@ void server_presize_slot(rgbdflow_server* s, ServerSlot& sl)
     q.xres_full = (unsigned)W;
     const int nb = std::max(1, std::min(s->cfg.max_batch, s->cfg.max_streams));
     std::vector<PairSpec> ps(nb, q);
-    const SlotNeed need = slot_need(ps, host_params(s->cfg.params), s->cfg.params.storage);
+    const SlotNeed need = slot_need(ps, host_params(s->cfg.params), s->cfg.params.storage, s->ctx->sms);
     const size_t other = other_slot_arenas(s, sl);
     if (sl.ctx->arena_cap < need.arena &&
         !(s->cfg.hbm_budget_bytes && s->resident_bytes + other + need.arena > s->cfg.hbm_budget_bytes))
@@ -2046,17 +2043,21 @@ extern "C" int rgbdflow_scene_flow_noalloc(const rgbdflow_pair* pair, const rgbd
         s.est = q.est_flow; s.out = q.flow_out;
         const std::vector<PairSpec> ps(1, s);
         const HostParams hp = host_params(*params);
-        Plan<float, float> P = make_plan<float, float>(ps, hp);
-        if (P.arena_bytes > kNoAllocScratchBytes)
-            throw ArgError(RGBDFLOW_ERR_BUDGET, "a " + std::to_string(q.W) + "x" + std::to_string(q.H) + " pair needs " +
-                                                    std::to_string(P.arena_bytes) + " workspace bytes; the static workspace holds " +
-                                                    std::to_string(kNoAllocScratchBytes) + " (one 320x240 pair)");
+        auto plan = [&](int sms) {
+            Plan<float, float> P = make_plan<float, float>(ps, hp, nullptr, sms);
+            if (P.arena_bytes > kNoAllocScratchBytes)
+                throw ArgError(RGBDFLOW_ERR_BUDGET, "a " + std::to_string(q.W) + "x" + std::to_string(q.H) + " pair needs " +
+                                                        std::to_string(P.arena_bytes) + " workspace bytes; the static workspace holds " +
+                                                        std::to_string(kNoAllocScratchBytes) + " (one 320x240 pair)");
+            return P;
+        };
+        Plan<float, float> P = plan(kPlanSms);  // an oversized pair is refused before a device is looked for
         int dev = 0;
         const cudaError_t ge = cudaGetDevice(&dev);
         if (ge != cudaSuccess) { cudaGetLastError(); throw ArgError(RGBDFLOW_ERR_NO_DEVICE, "no CUDA device"); }
         if (dev < 0 || dev >= kNoAllocMaxDevices) throw ArgError(RGBDFLOW_ERR_UNSUPPORTED, "device index above 63");
         const NoAllocDevice& d = noalloc_setup(dev);
-        P.sms = d.sms;
+        if (d.sms != P.sms) P = plan(d.sms);
         // no context's status word: the call's own, and what it says is in the flow
         P.status = (int*)(d.scratch + P.ctr_off) + 16;
         P.status_in_flow = true;
