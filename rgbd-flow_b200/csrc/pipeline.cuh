@@ -254,18 +254,24 @@ static inline int resident_fit(int W, int H, int kmax, int ctas)
     return 0;
 }
 
-// CTAs per item for k_level_bands on a step of n items, 0: not on it.  All clusters have to run together
-// (clusters of 16, 8, 4, 2 CTAs, one CTA an SM, of which the device holds 7, 16, 35, 74 at once), and a
+// What a plan depends on of the device.  As it stands here: one B200, for sizes asked without a device (others were
+// seen to hold 7, 15, 33 and 74).
+constexpr int kClusterSizes[4] = {16, 8, 4, 2};
+struct PlanDevice {
+    int sms = 148;                      // multiprocessors
+    int clusters[4] = {7, 16, 35, 74};  // clusters of kClusterSizes CTAs that run together, one CTA a multiprocessor
+};
+
+// CTAs per item for k_level_bands on a step of n items, 0: not on it.  All clusters have to run together, and a
 // band has to fit a CTA.  Among those the cheapest half-sweep: an update takes a scheduler 105 cycles a warp, its
 // chain about 200, a cluster barrier 330 more than a block's.
 template <class X>
-static int band_ctas(const std::vector<X>& items, int sms)
+static int band_ctas(const std::vector<X>& items, const PlanDevice& dev)
 {
-    static const int sizes[5][2] = {{16, 7}, {8, 16}, {4, 35}, {2, 74}, {1, 148}};
     int best = 0, best_cost = 1 << 30;
-    for (const auto& q : sizes) {
-        const int C = q[0];
-        bool fits = (int)items.size() <= q[1] && (int)items.size() * C <= sms;
+    for (int q = 0; q < 5; q++) {
+        const int C = q < 4 ? kClusterSizes[q] : 1;
+        bool fits = (int)items.size() <= (q < 4 ? dev.clusters[q] : dev.sms) && (int)items.size() * C <= dev.sms;
         int most = 0;
         for (const auto& x : items) {
             const int P = band_rows(x.H, C) * ((x.W + 1) / 2);
@@ -276,6 +282,14 @@ static int band_ctas(const std::vector<X>& items, int sms)
         if (fits && cost < best_cost) { best = C; best_cost = cost; }
     }
     return best;
+}
+// (a device of so many multiprocessors, grouped as a B200's)
+template <class X>
+static int band_ctas(const std::vector<X>& items, int sms)
+{
+    PlanDevice dev;
+    dev.sms = sms;
+    return band_ctas(items, dev);
 }
 
 // Iterations between the exchanges of the resident SOR, for the items of one step: a larger K exchanges less
@@ -649,16 +663,15 @@ static inline std::vector<SorLaunch> sor_schedule(int nSOR, int K, int period, i
     return v;
 }
 
-// sms: the device's multiprocessors, which decide what a step's SOR can keep resident.
-constexpr int kPlanSms = 148;  // a B200's, for sizes asked without a device
+// dev: what of a step's SOR can be resident together.
 template <class T, class S>
 static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams& hp, const TuneTable* tune = nullptr,
-                            int sms = kPlanSms)
+                            const PlanDevice& dev = PlanDevice())
 {
     if (!sor_tunable(hp)) tune = nullptr;
     Plan<T, S> P;
     P.hp = hp;
-    P.sms = sms;
+    P.sms = dev.sms;
     P.n = (int)pairs.size();
     P.kind = pairs.empty() ? 0 : pairs[0].kind;
     for (const auto& p : pairs) {
@@ -1014,7 +1027,7 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         P.step_tuned.push_back(ch != nullptr);
         const bool strips = ch ? ch->strip != 0 : strip_px >= (hp.strip_min_px > 0 ? hp.strip_min_px : 2000000L);
         std::vector<int> res_items;
-        const int band_c = regs && hp.res_k == 0 ? band_ctas(items, ctas) : 0;
+        const int band_c = regs && hp.res_k == 0 ? band_ctas(items, dev) : 0;
         int band_thr = 256;
         size_t band_smem = 0;
         for (auto& x : items) {
@@ -1441,6 +1454,36 @@ static void set_kernel_attrs()
         RF_CUDA(cudaFuncSetAttribute(k_sor_level_cluster_reg<T, S, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         RF_CUDA(cudaFuncSetAttribute(k_sor_level_cluster_reg<T, S, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     }
+}
+
+// The current device's PlanDevice: how many clusters run together depends on how its multiprocessors are grouped.
+static PlanDevice query_plan_device(int device)
+{
+    PlanDevice d;
+    RF_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
+    auto* const kernel = k_level_bands<float, kBandMax, true>;
+    RF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBandSmem));
+    RF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int q = 0; q < 4; q++) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kClusterSizes[q]);
+        cfg.blockDim = dim3(kBandMax);
+        cfg.dynamicSmemBytes = kBandSmem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClusterSizes[q];
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();  // no cluster of this size
+            n = 0;
+        }
+        d.clusters[q] = n;
+    }
+    return d;
 }
 
 // Whether configuration c fits shared memory for type T.

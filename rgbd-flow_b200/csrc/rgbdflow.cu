@@ -89,6 +89,17 @@ struct rgbdflow_ctx {
 
 namespace {
 
+// What plans depend on of a device (the current one), looked up once.
+const PlanDevice& plan_device(int device)
+{
+    static std::mutex mu;
+    static std::map<int, PlanDevice> known;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(device);
+    if (it == known.end()) it = known.emplace(device, query_plan_device(device)).first;
+    return it->second;
+}
+
 void drop_graphs(rgbdflow_ctx* c)
 {
     for (auto& kv : c->graphs) {
@@ -478,7 +489,7 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
     TuneTable& tt = ts.table[c->device & 63];
     const std::string bkey = plan_key(pairs, hp, (int)sizeof(T) * 10 + (int)sizeof(S));
     if (ts.complete[c->device & 63].count(bkey)) return;
-    const Plan<T, S> P0 = make_plan<T, S>(pairs, hp, &tt, c->sms);
+    const Plan<T, S> P0 = make_plan<T, S>(pairs, hp, &tt, plan_device(c->device));
     std::vector<int> todo;
     for (int sidx = 0; sidx < P0.Lmax; sidx++)
         if (!P0.step_tuned[sidx] && (P0.steps[sidx].n_sor || P0.steps[sidx].n_units)) todo.push_back(sidx);
@@ -506,7 +517,7 @@ void tune_sor(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const HostPar
         for (SorChoice cand : sor_candidates(P0, sidx)) {
             TuneTable one = tt;
             one.m[P0.step_keys[sidx]] = cand;
-            Plan<T, S> Pc = make_plan<T, S>(pairs, hp, &one, c->sms);
+            Plan<T, S> Pc = make_plan<T, S>(pairs, hp, &one, plan_device(c->device));
             ensure_arena(c, Pc.arena_bytes);
             bind_plan(Pc, c->arena);
             RF_CUDA(cudaMemcpy(c->arena + Pc.desc_off, Pc.desc.data(), Pc.desc_bytes, cudaMemcpyHostToDevice));
@@ -565,7 +576,7 @@ Plan<T, S> plan_for(rgbdflow_ctx* c, const std::vector<PairSpec>& pairs, const H
     tune_sor<T, S>(c, pairs, hp);
     TuneState& ts = tune_state();
     std::lock_guard<std::mutex> lk(ts.mu);
-    return make_plan<T, S>(pairs, hp, autotune_enabled() ? &ts.table[c->device & 63] : nullptr, c->sms);
+    return make_plan<T, S>(pairs, hp, autotune_enabled() ? &ts.table[c->device & 63] : nullptr, plan_device(c->device));
 }
 
 // Runs a batch through one graph launch.
@@ -1702,25 +1713,25 @@ void server_retire(rgbdflow_server* s, ServerSlot& sl)
 struct SlotNeed {
     size_t arena = 0, pin = 0;
 };
-SlotNeed slot_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, int sms)
+SlotNeed slot_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, const PlanDevice& dev)
 {
     // the storage type changes plane sizes only, not the descriptor count
     size_t arena = 0, desc = 0;
     if (storage == RGBDFLOW_STORE_FP16) {
-        const auto P = make_plan<float, __half>(ps, hp, nullptr, sms);
+        const auto P = make_plan<float, __half>(ps, hp, nullptr, dev);
         arena = P.arena_bytes; desc = P.desc_bytes;
     } else if (storage == RGBDFLOW_STORE_BF16) {
-        const auto P = make_plan<float, __nv_bfloat16>(ps, hp, nullptr, sms);
+        const auto P = make_plan<float, __nv_bfloat16>(ps, hp, nullptr, dev);
         arena = P.arena_bytes; desc = P.desc_bytes;
     } else {
-        const auto P = make_plan<float, float>(ps, hp, nullptr, sms);
+        const auto P = make_plan<float, float>(ps, hp, nullptr, dev);
         arena = P.arena_bytes; desc = P.desc_bytes;
     }
     return SlotNeed{arena, align_up(desc, 256) + sizeof(PairCtl) * ps.size()};
 }
-size_t slot_arena_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, int sms)
+size_t slot_arena_need(const std::vector<PairSpec>& ps, const HostParams& hp, int storage, const PlanDevice& dev)
 {
-    return slot_need(ps, hp, storage, sms).arena;
+    return slot_need(ps, hp, storage, dev).arena;
 }
 
 // Arena bytes of a batch for admission: the sum of its pairs' single-pair arenas (an upper bound:
@@ -1731,9 +1742,9 @@ size_t admit_need(rgbdflow_server* s, const std::vector<PairSpec>& ps, const Hos
     size_t tot = 0;
     for (const auto& q : ps) {
         const std::string key = std::to_string(q.W) + "x" + std::to_string(q.H) + (q.warm() ? "w" : "c") +
-                                std::to_string(s->cfg.params.storage) + "m" + std::to_string(s->ctx->sms) + plan_key({}, hp, 0);
+                                std::to_string(s->cfg.params.storage) + "d" + std::to_string(s->ctx->device) + plan_key({}, hp, 0);
         auto it = cache.find(key);
-        if (it == cache.end()) it = cache.emplace(key, slot_arena_need({q}, hp, s->cfg.params.storage, s->ctx->sms)).first;
+        if (it == cache.end()) it = cache.emplace(key, slot_arena_need({q}, hp, s->cfg.params.storage, plan_device(s->ctx->device))).first;
         tot += it->second;
     }
     return tot;
@@ -1754,7 +1765,7 @@ void server_presize_slot(rgbdflow_server* s, ServerSlot& sl)
     q.xres_full = (unsigned)W;
     const int nb = std::max(1, std::min(s->cfg.max_batch, s->cfg.max_streams));
     std::vector<PairSpec> ps(nb, q);
-    const SlotNeed need = slot_need(ps, host_params(s->cfg.params), s->cfg.params.storage, s->ctx->sms);
+    const SlotNeed need = slot_need(ps, host_params(s->cfg.params), s->cfg.params.storage, plan_device(s->ctx->device));
     const size_t other = other_slot_arenas(s, sl);
     if (sl.ctx->arena_cap < need.arena &&
         !(s->cfg.hbm_budget_bytes && s->resident_bytes + other + need.arena > s->cfg.hbm_budget_bytes))
@@ -1978,7 +1989,6 @@ __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 struct NoAllocDevice {
     char* scratch = nullptr;  // device address of g_noalloc_scratch on this device
-    int sms = 0;
 };
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1992,10 +2002,7 @@ const NoAllocDevice& noalloc_setup(int dev)
     if (d.scratch) return d;
     void* p = nullptr;
     RF_CUDA(cudaGetSymbolAddress(&p, g_noalloc_scratch));
-    int sms = 0;
-    RF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     set_kernel_attrs<float, float>();
-    d.sms = sms;
     d.scratch = (char*)p;
     return d;
 }
@@ -2043,21 +2050,18 @@ extern "C" int rgbdflow_scene_flow_noalloc(const rgbdflow_pair* pair, const rgbd
         s.est = q.est_flow; s.out = q.flow_out;
         const std::vector<PairSpec> ps(1, s);
         const HostParams hp = host_params(*params);
-        auto plan = [&](int sms) {
-            Plan<float, float> P = make_plan<float, float>(ps, hp, nullptr, sms);
-            if (P.arena_bytes > kNoAllocScratchBytes)
-                throw ArgError(RGBDFLOW_ERR_BUDGET, "a " + std::to_string(q.W) + "x" + std::to_string(q.H) + " pair needs " +
-                                                        std::to_string(P.arena_bytes) + " workspace bytes; the static workspace holds " +
-                                                        std::to_string(kNoAllocScratchBytes) + " (one 320x240 pair)");
-            return P;
-        };
-        Plan<float, float> P = plan(kPlanSms);  // an oversized pair is refused before a device is looked for
         int dev = 0;
-        const cudaError_t ge = cudaGetDevice(&dev);
-        if (ge != cudaSuccess) { cudaGetLastError(); throw ArgError(RGBDFLOW_ERR_NO_DEVICE, "no CUDA device"); }
+        const bool found = cudaGetDevice(&dev) == cudaSuccess;
+        if (!found) cudaGetLastError();
+        // an oversized pair is refused without a device too
+        Plan<float, float> P = make_plan<float, float>(ps, hp, nullptr, found ? plan_device(dev) : PlanDevice());
+        if (P.arena_bytes > kNoAllocScratchBytes)
+            throw ArgError(RGBDFLOW_ERR_BUDGET, "a " + std::to_string(q.W) + "x" + std::to_string(q.H) + " pair needs " +
+                                                    std::to_string(P.arena_bytes) + " workspace bytes; the static workspace holds " +
+                                                    std::to_string(kNoAllocScratchBytes) + " (one 320x240 pair)");
+        if (!found) throw ArgError(RGBDFLOW_ERR_NO_DEVICE, "no CUDA device");
         if (dev < 0 || dev >= kNoAllocMaxDevices) throw ArgError(RGBDFLOW_ERR_UNSUPPORTED, "device index above 63");
         const NoAllocDevice& d = noalloc_setup(dev);
-        if (d.sms != P.sms) P = plan(d.sms);
         // no context's status word: the call's own, and what it says is in the flow
         P.status = (int*)(d.scratch + P.ctr_off) + 16;
         P.status_in_flow = true;

@@ -34,7 +34,9 @@ int main()
                     q.f_full = 0.8f * s[0];
                     q.xres_full = s[0];
                 }
-                const Plan<float, float> P = make_plan<float, float>(pairs, params(10), nullptr, sms);
+                PlanDevice dev;
+                dev.sms = sms;
+                const Plan<float, float> P = make_plan<float, float>(pairs, params(10), nullptr, dev);
                 for (const auto& d : P.steps) {
                     const ResItem* ri = (const ResItem*)(P.desc.data() + d.res_items_off);
                     for (int i = 0; i < d.n_res; i++)
@@ -51,6 +53,25 @@ int main()
                     older += !d.regs;
                 }
             }
+    // a device that holds no clusters above a size (or none): smaller ones, or the launches of their own
+    for (int most : {8, 4, 2, 1}) {
+        PlanDevice dev;
+        for (int q = 0; q < 4; q++)
+            if (kClusterSizes[q] > most) dev.clusters[q] = 0;
+        for (const auto& s : sizes) {
+            std::vector<PairSpec> pairs(1);
+            pairs[0].W = s[0];
+            pairs[0].H = s[1];
+            pairs[0].f_full = 0.8f * s[0];
+            pairs[0].xres_full = s[0];
+            const Plan<float, float> P = make_plan<float, float>(pairs, params(10), nullptr, dev);
+            for (const auto& d : P.steps)
+                if (d.band_c > most) {
+                    std::printf("clusters of up to %d: bands of %d\n", most, d.band_c);
+                    return 1;
+                }
+        }
+    }
     if (!resident || !banded || !older) return 1;
     std::printf("ok plans\n");
     return 0;
