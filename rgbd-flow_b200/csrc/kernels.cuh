@@ -114,7 +114,6 @@ struct SorLaunch {
     int xout;          // whole-level kernel: ping-pong buffer that receives x (non-final inner iterations)
     int control;       // whole-level kernels: run the outer iteration's control after the fold (k_control's work)
     int n_checks;      // its convergence-check count
-    int masked;        // register kernels: the step is not finite, pixels outside the image are held at 0
 };
 
 template <class T, class S>

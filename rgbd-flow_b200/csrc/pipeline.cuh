@@ -1535,7 +1535,6 @@ static int enqueue_sor_regs(const Plan<T, S>& P, char* base, int sidx, cudaStrea
     L.final_fold = last;
     L.control = last;
     L.n_checks = n_checks;
-    L.masked = !std::isfinite(k.step);
     if (d.n_level) {
         L.xin = hh & 1;
         L.xout = L.xin ^ 1;
@@ -1547,10 +1546,11 @@ static int enqueue_sor_regs(const Plan<T, S>& P, char* base, int sidx, cudaStrea
     }
     if (!d.n_res) return launches;
     const ResItem* ri = (const ResItem*)(base + P.desc_off + d.res_items_off);
+    const bool overflow = !((double)k.step * P.hp.n_inner * P.hp.n_sor < 1e38);  // the unknowns may
     RF_PROF_B(pf, KC_SOR_LEVEL0 + lvl, st);
     for (int i = 0; i < d.n_res; i += kResItems) {
         const int n = std::min(kResItems, d.n_res - i);
-        launch_cooperative(k_sor_resident, std::min(P.sms, d.res_tiles), kResNT, st, ri + i, n, k, L,
+        launch_cooperative(overflow ? k_sor_resident<true> : k_sor_resident<false>, std::min(P.sms, d.res_tiles), kResNT, st, ri + i, n, k, L,
                            (unsigned)(outer * P.hp.n_inner + hh) * (unsigned)(P.hp.n_sor + 1),
                            P.hp.wait_polls >= 0 ? P.hp.wait_polls : resident_polls(n, P.hp.n_sor), P.status);
         launches++;

@@ -35,11 +35,12 @@ constexpr int kRegEx = 2 * 3 * 2 * 32;
 // One half-sweep (colour C) of a warp's block (its first row is even).  up / down: the other pixels' unknowns of the row
 // above / below the block, of this lane ([u, v, w], 64 elements apart); own: where this lane publishes.
 // Pixels outside the image have a system of zeros and start at 0, so they stay 0: 0 times a finite
-// neighbour adds nothing, and every unknown is finite while the step is (an update is clamped to
-// +-step around the old value, which also turns a NaN into one).  CHK: md takes the largest |change|
-// over the pixels of `mine` (bit 2 a + e: row a, column parity e); `in` (same bits) keeps pixels outside
-// the image at 0 whatever the step.
-template <int V, int C, bool CHK>
+// neighbour adds nothing, and every unknown is finite while the steps add up to a finite number (an update is
+// clamped to +-step around the old value, which also turns a NaN into one).  CHK: md takes the largest |change|
+// over the pixels of `mine` (bit 2 a + e: row a, column parity e).  MASK, for unknowns that may be infinite: `in` (same
+// bits) keeps pixels outside the image at 0, and what lies beside the region, with an edge of weight 0 (a shuffle
+// there gives the lane's own column), is taken as 0.
+template <int V, int C, bool CHK, bool MASK>
 __device__ __forceinline__ void reg_half_sweep(RegBlock<V>& b, const float* up, const float* down, float* own, float omega,
                                                float step, unsigned in, unsigned mine, float& md)
 {
@@ -66,18 +67,22 @@ __device__ __forceinline__ void reg_half_sweep(RegBlock<V>& b, const float* up, 
             }
             xu[v] = a > 0 ? b.x[a > 0 ? a - 1 : 0][e][v] : xu0[v];
             xd[v] = a < V - 1 ? b.x[a < V - 1 ? a + 1 : a][e][v] : xdV[v];
+            if (MASK && e == 0) xl[v] = (threadIdx.x & 31) != 0 ? xl[v] : 0.f;
+            if (MASK && e == 1) xr[v] = (threadIdx.x & 31) != 31 ? xr[v] : 0.f;
         }
         const float aL = e == 0 ? b.L[a] : b.R[a][0], wL = e == 0 ? b.Ls[a] : b.Rs[a][0];
         const float aU = a > 0 ? b.D[a > 0 ? a - 1 : 0][e] : b.U[e], wU = a > 0 ? b.Ds[a > 0 ? a - 1 : 0][e] : b.Us[e];
         sor_point_w<float>(b.c[a][e], aL, aU, b.R[a][e], b.D[a][e], wL, wU, b.Rs[a][e], b.Ds[a][e], xl, xu, xr, xd,
                            b.x[a][e], omega, step, nv);
-        if (CHK) {
-            const bool ok = (in >> (2 * a + e)) & 1, cnt = (mine >> (2 * a + e)) & 1;
+        if (MASK) {
+            const bool ok = (in >> (2 * a + e)) & 1;
 #pragma unroll
-            for (int v = 0; v < 3; v++) {
-                nv[v] = ok ? nv[v] : 0.f;
-                md = cnt ? fmaxf(md, fabsf(nv[v] - b.x[a][e][v])) : md;
-            }
+            for (int v = 0; v < 3; v++) nv[v] = ok ? nv[v] : 0.f;
+        }
+        if (CHK) {
+            const bool cnt = (mine >> (2 * a + e)) & 1;
+#pragma unroll
+            for (int v = 0; v < 3; v++) md = cnt ? fmaxf(md, fabsf(nv[v] - b.x[a][e][v])) : md;
         }
 #pragma unroll
         for (int v = 0; v < 3; v++) b.x[a][e][v] = nv[v];
@@ -284,7 +289,9 @@ static inline int resident_polls(int n_items, int n_sor)
     return p < (1 << 30) ? (int)p : 1 << 30;
 }
 
-// tag0: the launch's first tag less one; a launch uses at most n_sor of them.
+// tag0: the launch's first tag less one; a launch uses at most n_sor of them.  MASK: unknowns may overflow (a kernel of
+// its own: in one with the other, what it adds to the half-sweeps cost a solve 1.6 %).
+template <bool MASK>
 __global__ void __launch_bounds__(kResNT, 1)
 k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float> k, SorLaunch L, unsigned tag0,
                int polls, int* status)
@@ -370,14 +377,15 @@ k_sor_resident(const ResItem* __restrict__ items, int n_items, SolveConst<float>
             float md = 0.f;
 #pragma unroll 1
             for (int h = 0; h < 2 * nit; h++) {
-                if ((chk && h >= 2 * nit - 2) || L.masked) {
-                    // a check is of its own iteration, also where every one is masked
-                    const unsigned cnt = h >= 2 * nit - 2 ? mine : 0u;
-                    if (h & 1) reg_half_sweep<kResV, 1, true>(b, up, down, own, k.omega, k.step, in, cnt, md);
-                    else reg_half_sweep<kResV, 0, true>(b, up, down, own, k.omega, k.step, in, cnt, md);
+                // a check is of its own iteration (masked, every half-sweep takes the variant that can count)
+                const bool last = h >= 2 * nit - 2;
+                if (MASK || (chk && last)) {
+                    const unsigned cnt = last ? mine : 0u;
+                    if (h & 1) reg_half_sweep<kResV, 1, true, MASK>(b, up, down, own, k.omega, k.step, in, cnt, md);
+                    else reg_half_sweep<kResV, 0, true, MASK>(b, up, down, own, k.omega, k.step, in, cnt, md);
                 } else {
-                    if (h & 1) reg_half_sweep<kResV, 1, false>(b, up, down, own, k.omega, k.step, in, mine, md);
-                    else reg_half_sweep<kResV, 0, false>(b, up, down, own, k.omega, k.step, in, mine, md);
+                    if (h & 1) reg_half_sweep<kResV, 1, false, MASK>(b, up, down, own, k.omega, k.step, in, mine, md);
+                    else reg_half_sweep<kResV, 0, false, MASK>(b, up, down, own, k.omega, k.step, in, mine, md);
                 }
                 __syncthreads();
             }

@@ -35,3 +35,19 @@ def test_unclamped_step_stops_at_the_tile_sors_check(ctx, monkeypatch, W, H, tol
     tile = solve(ctx, W, H, 5, **over)
     assert any(0 < n < 200 for level in tile[1] for n in level[3])
     assert_same(regs, tile)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,omega,step,n_sor", [
+    (117, 93, 1.9, float("inf"), 100), (117, 93, 1.9, 3e38, 100), (64, 48, 1.9, float("inf"), 400), (64, 48, 1.9, 3e38, 100),
+    (200, 150, 1.9, 3e38, 400), (200, 150, 4.0, float("inf"), 100), (200, 150, 4.0, 1e37, 100)])
+def test_unknowns_that_overflow_do_so_as_the_tile_sors(ctx, monkeypatch, W, H, omega, step, n_sor):
+    """A relaxation that diverges until unknowns are infinite or NaN, on levels that end inside a tile and at a
+    tile's last column: nothing outside the image takes part."""
+    over = dict(max_flow_step=step, omega=omega, n_outer=2, n_sor=n_sor, sor_tol=0.0)
+    monkeypatch.setenv("RGBDFLOW_RESIDENT_K", "5")
+    regs = solve(ctx, W, H, 5, **over)
+    monkeypatch.setenv("RGBDFLOW_SOR_LEVEL", "0")
+    tile = solve(ctx, W, H, 5, **over)
+    assert np.nanmax(np.abs(tile[0])) > 1e30
+    assert_same(regs, tile)
