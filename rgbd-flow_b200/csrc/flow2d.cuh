@@ -312,7 +312,8 @@ __global__ void k_rhs(LevelBufs b, double alpha)
 // through L2 and more tasks than SMs.  Measured, one solve, device time: 320x240 85.8 ms (16), 73.1 (12), 65.8 (8),
 // 67.4 (6), 67.8 (4); 160x120 46.6, 39.4, 34.9, 34.2, 34.0.  Diagonal after diagonal over a cluster of 16 CTAs, a
 // cluster barrier a step and every value through L2, it was 637 ms at 320x240.
-constexpr int kPipeG = 8, kPipeThreads = 32 * (kPipeG + 2), kPipeAhead = 4, kPipePolls = 1 << 20;
+constexpr int kPipeG = 8, kPipeThreads = 32 * (kPipeG + 2), kPipeAhead = 4;
+constexpr int kPipePolls = 1 << 20;  // of a value, before a wait gives up
 
 struct PipeArgs {
     int W, H, NB;                 // level, bands
@@ -325,6 +326,7 @@ struct PipeArgs {
     int* conv;                    // first sweep below the threshold (0x7f7f7f7f: none yet; -1: a wait gave up)
     int zero_in;                  // the input is 0 (slot 0 is not read)
     int finish;
+    int polls;
     int* status;                  // 1: a bounded wait gave up
 };
 
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_sor_pipeline(PipeArgs a)
             };
             auto poll = [&](int t, double2 v) {
                 for (int k = 0; !pipe_ready(v); k++) {
-                    if (k >= kPipePolls) { gave_up = true; break; }
+                    if (k >= a.polls) { gave_up = true; break; }
                     if ((k & 15) == 15 && *(volatile int*)a.conv < (a.finish ? 0 : a.s0 + g * a.G)) { stop = true; break; }
                     v = pipe_load(at(t), true);
                 }

@@ -132,7 +132,7 @@ void check_status(rgbdflow_ctx* c)
     *c->pin_status = 0;
     RF_CUDA(cudaMemsetAsync(c->dev_status, 0, sizeof(int), c->stream));
     RF_CUDA(cudaStreamSynchronize(c->stream));
-    throw ArgError(RGBDFLOW_ERR_TIMEOUT, "a bounded device wait (grid barrier) gave up: the solve's results are not valid");
+    throw ArgError(RGBDFLOW_ERR_TIMEOUT, "a bounded device wait gave up: the solve's results are not valid");
 }
 
 void ensure_arena(rgbdflow_ctx* c, size_t need)
@@ -164,6 +164,13 @@ void ensure_pin(rgbdflow_ctx* c, size_t need)
     const size_t cap = align_up(need + need / 8, 1 << 20);
     RF_CUDA(cudaMallocHost(&c->pin, cap));
     c->pin_cap = cap;
+}
+
+// Polls after which the SOR's waits between thread blocks give up (-1: each kernel's own limit).
+int wait_polls()
+{
+    const char* e = std::getenv("RGBDFLOW_WAIT_POLLS");
+    return e ? std::max(0, std::atoi(e)) : -1;
 }
 
 HostParams host_params(const rgbdflow_params& p)
@@ -203,8 +210,7 @@ HostParams host_params(const rgbdflow_params& p)
     h.level_reg = e ? std::atoi(e) : 1;
     e = std::getenv("RGBDFLOW_RESIDENT_K");
     h.res_k = e ? std::atoi(e) : 0;
-    e = std::getenv("RGBDFLOW_WAIT_POLLS");
-    h.wait_polls = e ? std::max(0, std::atoi(e)) : -1;
+    h.wait_polls = wait_polls();
     h.fill_rounds = 253;  // round stamps are bytes: 0 valid, 1..253 rounds, 254 outside, 255 unfilled
     return h;
 }
@@ -796,6 +802,7 @@ static int enqueue_sor_pipeline(rgbdflow_ctx* c, const rgbdflow::f2d::LevelBufs&
     using namespace rgbdflow::f2d;
     const PipePlan plan = pipe_plan(b.W, b.H, nSOR, ws_bytes);
     if (!plan.groups) throw ArgError(RGBDFLOW_ERR_INTERNAL, "2-D SOR work space too small");
+    const int limit = wait_polls(), polls = limit >= 0 ? limit : kPipePolls;
     int launches = 0;
     RF_CUDA(cudaMemsetAsync(ctl + 1, 0x7f, sizeof(int), st));
     for (int s0 = 0; s0 < nSOR;) {
@@ -816,6 +823,7 @@ static int enqueue_sor_pipeline(rgbdflow_ctx* c, const rgbdflow::f2d::LevelBufs&
         a.sweep = (ulonglong2*)(ws + img_bytes + bnd_bytes);
         a.conv = ctl + 1;
         a.status = ctl;
+        a.polls = polls;
         a.zero_in = s0 == 0;
         if (s0) RF_CUDA(cudaMemcpyAsync(ws, ws + (size_t)plan.groups * plan.img, plan.img, cudaMemcpyDeviceToDevice, st));
         RF_CUDA(cudaMemsetAsync(ws + plan.img, 0xff, img_bytes - plan.img + bnd_bytes, st));
@@ -1007,7 +1015,7 @@ static void run_flow2d(rgbdflow_ctx* c, const uint8_t* bgr1, const uint8_t* bgr2
     RF_CUDA(cudaMemcpyAsync(&status, ctl, sizeof(status), cudaMemcpyDeviceToHost, st));
     RF_CUDA(cudaStreamSynchronize(st));
     c->last_launches = launches;
-    if (status) throw ArgError(RGBDFLOW_ERR_INTERNAL, "2-D SOR ran out of its step bound");
+    if (status) throw ArgError(RGBDFLOW_ERR_TIMEOUT, "a bounded device wait of the 2-D SOR gave up: the solve's results are not valid");
     for (size_t z = 0; z < N0; z++) {
         flow_out[z * 2] = (float)u[z];
         flow_out[z * 2 + 1] = (float)v[z];

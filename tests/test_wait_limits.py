@@ -107,3 +107,18 @@ def test_a_lost_wait_of_the_allocation_free_solve_is_in_its_flow(monkeypatch, K)
     assert np.isnan(flow()).all()
     monkeypatch.delenv("RGBDFLOW_WAIT_POLLS")
     np.testing.assert_array_equal(flow(), before)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_inner", [1, 2])
+def test_2d_sor_reports_lost_waits(ctx, monkeypatch, n_inner):
+    """Several bands and groups of sweeps, so that tasks wait for others' values; later solves run as before."""
+    p = pair(64, 80, 3)
+    prm = rf.flow2d_params(n_outer=2, n_inner=n_inner, n_sor=40)
+    before = ctx.optical_flow_2d(p["bgr1"], p["bgr2"], prm)
+    monkeypatch.setenv("RGBDFLOW_WAIT_POLLS", "0")
+    with pytest.raises(rf.RgbdFlowError) as e:
+        ctx.optical_flow_2d(p["bgr1"], p["bgr2"], prm)
+    assert e.value.code == TIMEOUT
+    monkeypatch.delenv("RGBDFLOW_WAIT_POLLS")
+    np.testing.assert_array_equal(ctx.optical_flow_2d(p["bgr1"], p["bgr2"], prm), before)
