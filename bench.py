@@ -14,7 +14,8 @@ run N replicas (weak scaling, no collective on the data path).
              contexts in rotation), every step's host->device inputs and device->host flows inside
              the timed region
   plain      one pair per call (the drop-in solve): pairs/s and p50 / p99 latency
-  roofline   the dominant kernel (red-black SOR) from a profiled pass of the same workload
+  roofline   the dominant kernel (red-black SOR) from a profiled pass of the same workload, against the
+             FP32 issue rate that bounds it
   cpu_baseline  the CPU restatement of the reference (oracle, all host threads) on one pair
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--batch B] [--impl ours|reference]
@@ -37,16 +38,21 @@ METRIC = "640×480 pairs/s & p99 latency, served+batched vs plain GPU at matched
 W, H = 640, 480
 
 
+# FP32 instructions of a pixel update: three rows of 6 multiply-adds, 3 products, 3 additions, a minimum and a maximum
+SOR_INSTRUCTIONS = 42
+
+
 def peaks():
+    """The measured copy bandwidth and the highest SM clock of this kind of GPU."""
     try:
         m = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
-        return float(m["hbm_gbs"]), "measured"
+        return {"hbm_gbs": float(m["hbm_gbs"]), "sm_max_mhz": float(m["sm_max_mhz"])}
     except Exception:
-        return 6650.0, "fallback"
+        return {"hbm_gbs": 6650.0, "sm_max_mhz": 1965.0}
 
 
 def ncu_traffic():
-    """DRAM bytes of a level-0 strip-SOR launch per pair, from the committed ncu summary
+    """DRAM bytes of a level-0 launch of the register SOR per pair, from the committed ncu summary
     (profiles/sor_traffic.json), if present."""
     try:
         d = json.load(open(os.path.join(ROOT, "profiles", "sor_traffic.json")))
@@ -598,31 +604,34 @@ def main():
                       "inputs from page-locked host memory, solves, and downloads its flows; one step's transfers "
                       "overlap the other contexts' solves" % LANES}
 
-    # ---- roofline of the dominant kernel from a profiled pass of the same workload: the SOR of
-    # the 640x480 level (the strip kernel), algorithmic bytes / live CUDA-event time
+    # ---- roofline of the dominant kernel from a profiled pass of the same workload: the SOR of the 640x480
+    # level from registers.  It keeps its data on chip, so what bounds it is instruction issue: the FP32
+    # instructions of the executed pixel updates / live CUDA-event time, against one a lane and clock
     ctx.profile(1)
     for _ in range(2):
         ctx.scene_flow_batch_device(dev, prm)
     torch.cuda.synchronize()
     kst = ctx.profile_read()
     ctx.profile(0)
-    peak, peak_kind = peaks()
-    n0, ms0, b0 = kst.get("sor_level0", (0, 0.0, 0.0))
-    n_sor, sor_ms, sor_bytes = kst.get("sor", (0, 0.0, 0.0))
-    achieved = b0 / (ms0 / 1e3) / 1e9 if ms0 > 0 else 0.0
+    stats = ctx.scene_flow_batch(hp, prm)[1]
+    iters = sum(st.sor_iters[0][o] for st in stats for o in range(st.outer_iters[0]))
+    n0, ms0, _ = kst.get("sor_level0", (0, 0.0, 0.0))
+    n_sor, sor_ms, _ = kst.get("sor", (0, 0.0, 0.0))
+    achieved = 2 * iters * W * H * SOR_INSTRUCTIONS / (ms0 / 1e3) / 1e12 if ms0 > 0 else 0.0
+    sms, mhz = torch.cuda.get_device_properties(local).multi_processor_count, peaks()["sm_max_mhz"]
+    peak = sms * 128 * mhz * 1e6 / 1e12
     tr = ncu_traffic()
     tot_ms = sum(v[1] for k, v in kst.items() if not k.startswith("sor_level"))
-    roofline = {"kernel": "k_sor_strip: red-black SOR of the 640x480 level over 64-column strips, rows streamed "
-                          "through a shared-memory ring, 5 sweeps per launch",
-                "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "peak_source": peak_kind,
+    roofline = {"kernel": "k_sor_resident: red-black SOR of the 640x480 level from registers, with its fold (k_sor_fold)",
+                "bound": "fp32 issue", "achieved": achieved, "peak": peak, "unit": "T FP32 instructions/s", "frac": achieved / peak,
+                "peak_source": "%d SMs x 128 lanes x %d MHz" % (sms, mhz),
                 "traffic": (tr["dram_bytes_per_launch_per_pair"] * B if tr else None),
-                "algorithmic_bytes_per_launch": b0 / max(n0, 1),
+                "traffic_gbs": (tr["dram_bytes_per_launch_per_pair"] * B * n0 / (ms0 / 1e3) / 1e9 if tr and ms0 > 0 else None),
+                "hbm_peak_gbs": peaks()["hbm_gbs"],
+                "us_per_pair_iteration": 1e3 * ms0 / (2 * iters) if iters else None,
                 "avg_launch_us": 1e3 * ms0 / max(n0, 1), "launches": n0,
                 "share_of_device_time": ms0 / tot_ms if tot_ms else None,
-                "all_sor_levels": {"achieved_gbs": sor_bytes / (sor_ms / 1e3) / 1e9 if sor_ms > 0 else 0.0,
-                                   "frac": (sor_bytes / (sor_ms / 1e3) / 1e9) / peak if sor_ms > 0 else 0.0,
-                                   "share_of_device_time": sor_ms / tot_ms if tot_ms else None},
+                "all_sor_levels": {"share_of_device_time": sor_ms / tot_ms if tot_ms else None},
                 "kernel_ms": {k: round(v[1], 3) for k, v in kst.items()}}
     if tr:
         roofline["traffic_note"] = tr.get("note", "")
