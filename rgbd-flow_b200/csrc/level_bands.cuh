@@ -83,8 +83,9 @@ __device__ __forceinline__ void mbar_expect(unsigned mbar, int bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
-// Waits (`polls` tries) for the phase of the given parity; false: it gave up.
-constexpr int kBandPolls = 1 << 20;
+// Waits (`polls` tries) for the phase of the given parity; false: it gave up.  A try that fails has blocked for 4 us
+// (measured), so that a wait gives up after a second.
+constexpr int kBandPolls = 1 << 18;
 __device__ __forceinline__ bool mbar_wait(unsigned mbar, int parity, int polls)
 {
     for (int p = 0; p < polls; p++) {

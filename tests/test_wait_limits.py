@@ -122,3 +122,13 @@ def test_2d_sor_reports_lost_waits(ctx, monkeypatch, n_inner):
     assert e.value.code == TIMEOUT
     monkeypatch.delenv("RGBDFLOW_WAIT_POLLS")
     np.testing.assert_array_equal(ctx.optical_flow_2d(p["bgr1"], p["bgr2"], prm), before)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc to compile the probe")
+def test_level_bands_waits_take_a_second(tmp_path):
+    exe = str(tmp_path / "wait_time_check")
+    subprocess.run(["nvcc", "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                    os.path.join(HERE, "cpp", "wait_time_check.cu")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
