@@ -1890,6 +1890,8 @@ k_sor_level_reg(const LevelItem<T, S>* items, const int* which, SolveConst<T> k,
 // so every CTA takes the same decision.  At the end x goes to global memory and, for the fold, each
 // 32 x 32 tile's u += x and statistic partial is taken by one CTA in the tile kernels' order, so
 // results equal the tile kernel's bit for bit, as the one-CTA whole-level kernel's do.
+// FP32 steps whose levels all fit the device's registers do not come here (sor_from_registers): these two cluster
+// kernels serve FP64, steps with a level that does not fit, and SOR settings given explicitly.
 // Shared layout: 15 planes of [B + 2 rows][2 colours][hwp + 2 positions], padding zero.
 template <class T> __host__ __device__ constexpr size_t level_cluster_smem_bytes(int B, int hwp)
 {

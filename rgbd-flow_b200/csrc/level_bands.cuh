@@ -15,6 +15,7 @@
 //   10x7, 1 CTA    370; SOR 22 K, linearisation 8 K, fold 0.8 K
 //   80x60, 16      840; SOR 50 K, linearisation 11 K, fold 5 K (a cluster barrier a half-sweep: 1060)
 //   160x120, 16   1330; SOR 79 K, linearisation 22 K, fold 11 K (1720)
+// (the form for 640 threads, which 160x120 takes, has 96 registers a thread and spills: 188 bytes of stores, 224 of loads)
 // against 60, 120 and 120 K for the SOR alone as launches of k_sor_level_reg and k_sor_resident, and 25 to 40 us an
 // outer iteration for the rest.  A half-sweep of 80x60 is 370 cycles of update and block barrier and the way of the
 // neighbours' rows (about 470).  A 160x120 solve 1.17 -> 0.89 ms, one of 320x240 without allocations 1.63 -> 1.30.

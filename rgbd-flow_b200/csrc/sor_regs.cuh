@@ -196,9 +196,11 @@ __device__ __forceinline__ void reg_block_store(const RegBlock<V>& b, float* x, 
 // in, so that all take the same decision.  Launched cooperatively (the CTAs wait for one another), every
 // wait bounded.
 //
-// What bounds it: the half-sweeps (0.65 us; 105 cycles of a scheduler per warp and pixel update, of which
-// the FP32 operations' register reads take 70), then the exchange (1.8 us: half of it the way through L2; by
-// flags -- store, barrier, fence, flag; poll with acquire loads, barrier, load -- it took 4.8 us).
+// What bounds it: the half-sweeps (0.65 us; 106 cycles of a scheduler per warp and pixel update, for which a launch
+// executes 91 instructions, load and exchange included, 42 of them the update's arithmetic), then the exchange (1.8 us:
+// half of it the way through L2; by flags -- store, barrier, fence, flag; poll with acquire loads, barrier, load -- it
+// took 4.8 us).  Of the 168 registers a thread may have 96 bytes more are in local memory (spill stores 156 bytes, loads
+// 216).
 // Measured, 30 iterations of one level (one pair): 640x480 91 us (tile SOR 261), 320x240 64 (108), 160x120 63
 // and 80x60 63 (cluster whole-level kernel 126 and 105); 16 pairs: 640x480 15.4 -> 9.1 ms of SOR a solve (strip
 // SOR), 320x240 3.3 -> 1.6 (strips), 160x120 0.81 -> 0.44 (cluster).  Levels of more than 148 tiles (about
