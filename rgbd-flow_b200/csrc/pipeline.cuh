@@ -1585,7 +1585,7 @@ static int enqueue_level(const Plan<T, S>& P, char* base, int sidx, cudaStream_t
         launches++;
     }
     if constexpr (sizeof(T) == 4)
-        if (d.band_c) {
+        if (d.band_c && P.hp.n_outer > 0) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(d.n_items * d.band_c);
             cfg.blockDim = dim3(d.band_threads);

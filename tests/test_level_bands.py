@@ -65,3 +65,13 @@ def test_level_bands_of_a_ragged_batch(ctx, monkeypatch, n):
     for q, b in list(zip(pairs, batch))[:9]:
         np.testing.assert_array_equal(ctx.scene_flow_two_frames(q["cam"], q["bgr1"], q["depth1"], q["bgr2"], q["depth2"], prm,
                                                                 stats=False), b)
+
+
+@pytest.mark.gpu
+def test_no_outer_iterations_launch_nothing(ctx, monkeypatch):
+    a = args(160, 120, 7, n_outer=0)
+    bands = ctx.scene_flow_two_frames(*a, stats=False)
+    launches = ctx.last_launch_count()
+    monkeypatch.setenv("RGBDFLOW_SOR_LEVEL", "0")
+    np.testing.assert_array_equal(ctx.scene_flow_two_frames(*a, stats=False), bands)
+    assert ctx.last_launch_count() == launches
