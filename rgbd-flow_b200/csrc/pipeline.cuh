@@ -582,7 +582,7 @@ struct Plan {
         size_t clus_smem;
         int clus_kp;  // > 0: the cluster items run on k_sor_level_cluster_reg with this many positions a thread
         size_t res_items_off; int n_res;      // k_sor_resident: ResItem per item
-        int res_k, res_tiles;                 // iterations between exchanges, tiles of the step
+        int res_k, res_tiles;                 // iterations between exchanges (the items' most), tiles of the step
         int n_fold;                           // blocks of its fold (32 x 32 tiles)
         bool regs;                            // the step's items all run from registers
         int band_c, band_threads;             // > 0: the step runs on k_level_bands, band_c CTAs an item
@@ -1131,7 +1131,7 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
         d.res_k = 0;
         d.res_tiles = 0;
         d.n_fold = 0;
-        if (!res_items.empty()) d.res_k = hp.res_k > 0 ? std::min(hp.res_k, kResMaxK) : resident_k(items, res_items, ctas);
+        const int most_k = res_items.empty() ? 0 : hp.res_k > 0 ? std::min(hp.res_k, kResMaxK) : resident_k(items, res_items, ctas);
         for (int i : res_items) {
             const auto& x = items[i];
             ResItem m;
@@ -1144,7 +1144,8 @@ static Plan<T, S> make_plan(const std::vector<PairSpec>& pairs, const HostParams
                 if ((size_t)(z < 6 ? x.x[z / 3][z % 3] : x.sys[z - 6]) != (size_t)m.x + sizeof(float) * m.stride * z)
                     throw std::logic_error("increment and system planes not evenly spaced");
             m.W = x.W; m.H = x.H; m.hw = x.hwp;
-            m.K = resident_fit(x.W, x.H, d.res_k, ctas);
+            m.K = resident_fit(x.W, x.H, most_k, ctas);
+            d.res_k = std::max(d.res_k, m.K);
             m.nx = res_tiles(x.W, kResCols, m.K);
             m.ny = res_tiles(x.H, kResRows, m.K);
             d.res_tiles += m.nx * m.ny;

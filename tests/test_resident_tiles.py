@@ -82,3 +82,19 @@ def test_register_sor_batch_larger_than_the_device(ctx, monkeypatch):
     for q, b in zip(pairs, batch):
         np.testing.assert_array_equal(ctx.scene_flow_two_frames(q["cam"], q["bgr1"], q["depth1"], q["bgr2"], q["depth2"], prm,
                                                                 stats=False), b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(608, 456), (200, 152)])
+def test_listing_names_the_exchanges_that_run(ctx, W, H):
+    """The iterations between exchanges at which the level's tiles fit the device, not the most there may be."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    p = pair(W, H, 1)
+    prm = rf.benchmark_params(W, n_outer=1)
+    prm.min_width = W
+    cam = rf.CameraParams.make(W, H, p["cam"].f, p["cam"].cx, p["cam"].cy)
+    ctx.scene_flow_two_frames(cam, p["bgr1"], p["depth1"], p["bgr2"], p["depth2"], prm, stats=False)
+    tiles = lambda K: -(-(W - 4 * K) // (64 - 4 * K)) * -(-(H - 4 * K) // (48 - 4 * K))  # noqa: E731
+    K = max(k for k in range(1, 6) if tiles(k) <= sms)
+    assert "f%dx%d*1, registers, exchange every %d;" % (W, H, K) in rf.autotune_describe(0)
