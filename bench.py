@@ -315,7 +315,7 @@ def run_precision(ctx, rf, torch, stream, dev, pairs, args):
         torch.cuda.synchronize()
         kst = ctx.profile_read()
         ctx.profile(0)
-        gbs = {k: kst[k][2] / (kst[k][1] / 1e3) / 1e9 for k in ("sor", "linearize") if k in kst and kst[k][1] > 0}
+        gbs = {k: kst[k][2] / (kst[k][1] / 1e3) / 1e9 for k in ("linearize",) if k in kst and kst[k][1] > 0}
         out[name] = {"pairs_per_s": 1e3 * len(dev) / ms,
                      "epe_vs_fp64_mm": {"mean": 1e3 * float(np.mean([e[0] for e in e64])),
                                         "max": 1e3 * float(np.max([e[1] for e in e64]))},

@@ -1837,7 +1837,10 @@ static int enqueue_solve(const Plan<T, S>& P, char* base, cudaStream_t st, Prof*
 //        fold u += x (u read and written, 24 B).
 //   linearisation: per level pixel and execution, 20 input values (5 + 5 features, 2 depths,
 //        3 flow, 5 weights; the 12 feature/depth values in the storage type) plus the 12-float
-//        system written.
+//        system written; not of levels that k_level_bands solves, whose linearisation is in the
+//        SOR's time.
+// The register kernels read a system once an inner iteration or not at all: for them the SOR's bytes are a count of
+// iterations, not of traffic.
 template <class T, class S>
 static void executed_bytes(const Plan<T, S>& P, const PairCtl* ctl, double* sor_bytes, double* lin_bytes,
                            double* sor_level = nullptr)
@@ -1855,7 +1858,7 @@ static void executed_bytes(const Plan<T, S>& P, const PairCtl* ctl, double* sor_
                 const double b = N * (ctl[p].sor_exec[k][o] * 72.0 * sizeof(T) / 4.0 + 24.0 * sizeof(T) / 4.0);
                 *sor_bytes += b;
                 if (sor_level) sor_level[k] += b;
-                *lin_bytes += N * lin_px * P.hp.n_inner;
+                if (!P.steps[P.Lmax - 1 - k].band_c) *lin_bytes += N * lin_px * P.hp.n_inner;
             }
         }
 }

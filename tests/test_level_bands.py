@@ -75,3 +75,15 @@ def test_no_outer_iterations_launch_nothing(ctx, monkeypatch):
     monkeypatch.setenv("RGBDFLOW_SOR_LEVEL", "0")
     np.testing.assert_array_equal(ctx.scene_flow_two_frames(*a, stats=False), bands)
     assert ctx.last_launch_count() == launches
+
+
+@pytest.mark.gpu
+def test_profile_counts_the_linearisation_of_its_own_launches(ctx):
+    """320x240 is linearised by k_linearize, the levels below it inside k_level_bands, in the SOR's time."""
+    a = args(320, 240, 7)
+    a[-1].min_width = 20
+    ctx.profile(1)
+    _, st = ctx.scene_flow_two_frames(*a)
+    kst = ctx.profile_read()
+    ctx.profile(0)
+    assert kst["linearize"][2] == 320 * 240 * 128.0 * st.outer_iters[0]
